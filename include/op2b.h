@@ -30,8 +30,9 @@ enum { OP2B_STRATEGY_AUTO = 0, OP2B_STRATEGY_GATHER = 1, OP2B_STRATEGY_COLOURED 
 /* How global OP_INC reductions (op_arg_gbl ... OP_INC) are summed.
  *  TREE : fixed-shape tree (per-thread, warp shuffle, per-block, one final
  *         block); deterministic run to run.
- *  SEQ  : element order, one addition at a time, exactly as op_seq.h does;
- *         bit-identical to the reference, at the cost of a serial pass. */
+ *  SEQ  : element order, one rounding per addition, exactly as op_seq.h does;
+ *         bit-identical to the reference, at the cost of two more launches
+ *         (about 50 us for 720k values). */
 enum { OP2B_REDUCE_TREE = 0, OP2B_REDUCE_SEQ = 1 };
 
 /* Kernel-variant knobs, used by the tuner and by experiments; returns the

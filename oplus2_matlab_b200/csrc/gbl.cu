@@ -11,14 +11,16 @@
 
 #include <algorithm>
 
+#include "launch.cuh"
 #include "loops.h"
+#include "seq_sum.cuh"
 
 namespace op2b {
 
 namespace {
 constexpr int kSlots = 4096;
 struct RedState {
-  char *dev = nullptr;  // [2 x kMaxRedBlocks x 8] partials | ticket (256 B)
+  char *dev = nullptr;  // [2 x kMaxRedBlocks x 8] partials | tickets (256 B)
   // result slots in mapped pinned host memory: the last block of a reduction
   // stores the result where the host reads it, so delivery needs no copy
   char *host = nullptr;
@@ -108,16 +110,38 @@ int red_new_slot() {
   return S.next_slot++;
 }
 
+// the values, then seq_sum's tables: a sum, two pairs and a binade per tile of
+// values (at least 4 bytes each), two pairs per run
+static size_t seq_table_offset(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
+
 void *red_seq_buffer(size_t bytes) {
   RedState &S = rs();
   if (bytes > S.seq_bytes) {
     OP2B_CUDA(cudaStreamSynchronize(rt().stream));
     dev_free(S.seq);
-    S.seq = dev_alloc(bytes);
-    S.seq_bytes = bytes;
+    S.seq = dev_alloc(seq_table_offset(bytes) +
+                      (bytes / 4 / kSeqTile + 2) *
+                          (sizeof(double) + (1 + kSeqRuns) * sizeof(SeqTwo<double>) + 8));
+    S.seq_bytes = S.seq ? bytes : 0;
   }
   return S.seq;
 }
+
+template <class T>
+void seq_sum(const T *v, long long n, T init, T *out, const int *order, int w) {
+  const int ntile = (int)std::max(1LL, (n + kSeqTile - 1) / kSeqTile);
+  char *tab = (char *)v + seq_table_offset(sizeof(T) * (size_t)n);
+  double *tsum = (double *)tab;
+  SeqTwo<T> *tiles = (SeqTwo<T> *)(tsum + ntile), *runs = tiles + ntile;
+  int *binade = (int *)(runs + (size_t)ntile * kSeqRuns);
+  const SeqVals<T> a{v, n, order, w};
+  cudaStream_t s = rt().stream;
+  launch_pdl(k_seq_tile_sums<T>, ntile, kSeqThreads, 0, s, a, tsum);
+  launch_pdl(k_seq_fold<T>, ntile, kSeqThreads, 0, s, a, init, ntile, (const double *)tsum, tiles,
+             runs, binade, red_ticket() + 1, out);
+}
+template void seq_sum<float>(const float *, long long, float, float *, const int *, int);
+template void seq_sum<double>(const double *, long long, double, double *, const int *, int);
 
 int red_grid(long long n, int threads) {
   long long want = (n + threads - 1) / threads;

@@ -306,8 +306,7 @@ static void jac_update_t(char const *name, op_set set, const op_arg *args,
                (float *)args[1].dat->data_d, (float *)args[2].dat->data_d, alpha, seqbuf, ss, sm,
                red_ticket());
     if (seq)
-      k_seq_sum<float><<<1, 32, 0, s>>>(seqbuf, n, *(const float *)args[3].data, r_sum,
-                                        perm_old2new_dev(set), 1);
+      seq_sum<float>(seqbuf, n, *(const float *)args[3].data, r_sum, perm_old2new_dev(set), 1);
   }
   std::vector<GblRequest> rq{GblRequest{args[3].data, slot_sum, OP_INC, GBL_F32, seq},
                              GblRequest{args[4].data, slot_max, OP_MAX, GBL_F32, false}};
@@ -564,8 +563,7 @@ bool run_jac_step(char const *uname, op_set uset, const op_arg *ua, char const *
                (const float *)r->data_d, (const float *)du->data_d, (const float *)u->data_d,
                alpha, beta, u_out, du_out, seqbuf, ss, sm, red_ticket());
     if (seq)
-      k_seq_sum<float><<<1, 32, 0, s>>>(seqbuf, n, *(const float *)ua[3].data, r_sum,
-                                        perm_old2new_dev(uset), 1);
+      seq_sum<float>(seqbuf, n, *(const float *)ua[3].data, r_sum, perm_old2new_dev(uset), 1);
   }
   if (error_pending()) return true;
   flip(u, capturing);

@@ -47,6 +47,10 @@ unsigned *red_ticket();
 void *red_slot_ptr(int slot);    // 8-byte device slot
 int red_new_slot();
 void *red_seq_buffer(size_t bytes);  // scratch for SEQ-mode contributions
+// *out = init + v[0] + v[1] + ... + v[n-1], added in that order (value j of a
+// renumbered set: see SeqVals); v is red_seq_buffer's
+template <class T>
+void seq_sum(const T *v, long long n, T init, T *out, const int *order, int w);
 void red_finish(const std::vector<GblRequest> &reqs);
 // the same, waiting only for the work up to the event (not deferred mode)
 void red_finish_after(cudaEvent_t done, const std::vector<GblRequest> &reqs);
