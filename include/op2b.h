@@ -20,10 +20,13 @@ extern "C" {
  *             in ascending (element, argument) order, which is exactly the
  *             order of the reference's sequential op_seq.h back-end, so the
  *             results are bit-identical to it.  No colouring, no atomics.
- *  COLOURED : the two-level colouring of op_plan (blocks staged in shared
- *             memory, increments applied in thread-colour order, blocks
- *             launched colour by colour).  Deterministic; summation order
- *             differs from op_seq.h, as in the reference's CUDA/OpenMP code.
+ *  COLOURED : the two-level colouring of op_plan: a block's increments of a
+ *             target added in thread-colour order, the blocks' sums in block
+ *             colour order (res_calc by two passes over lists in that order,
+ *             knob "coloured_fold"; the others blocks staged in shared
+ *             memory and launched colour by colour).  Deterministic; summation
+ *             order differs from op_seq.h, as in the reference's CUDA/OpenMP
+ *             code.
  *  AUTO     : per loop, the faster of the two as measured by the tuner. */
 enum { OP2B_STRATEGY_AUTO = 0, OP2B_STRATEGY_GATHER = 1, OP2B_STRATEGY_COLOURED = 2 };
 
@@ -59,6 +62,9 @@ enum { OP2B_REDUCE_TREE = 0, OP2B_REDUCE_SEQ = 1 };
  *                   the res that follows it as one launch ("jac_tile_nodes"
  *                   the tile size, 0 automatic; "jac_step_threads" 512,
  *                   1024 or 256 per CTA); 0: two launches
+ *   "coloured_fold" 1 (default): COLOURED res_calc [+ bres_calc ...] as the
+ *                   flux pass and a per-cell fold in the plan's order; 0: one
+ *                   launch per block colour
  *   "known_zero"    1 (default): the res_calc chain neither reads nor
  *                   rewrites res when res is known to hold zeros
  *                   (op2b_res_skips); 0: it always reads res

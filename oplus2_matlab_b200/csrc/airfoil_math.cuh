@@ -161,4 +161,22 @@ __device__ __forceinline__ void add_listed(T r[4], int k, const T f[4]) {
   }
 }
 
+// the same for a list in the order of the two-level colouring (entry = index
+// << 2 | last of its block << 1 | negate; -1: none).  A block's increments of
+// the cell gather in acc from +0, each as 0 + f or 0 - f, and its last adds
+// the block's sum to r: the additions of the block kernels, in their order
+template <class T>
+__device__ __forceinline__ void add_coloured(T r[4], T acc[4], int k, const T f[4]) {
+  if (k < 0) return;
+#pragma unroll
+  for (int d = 0; d < 4; d++) acc[d] += (k & 1) ? T(0) - f[d] : T(0) + f[d];
+  if (k & 2) {
+#pragma unroll
+    for (int d = 0; d < 4; d++) {
+      r[d] += acc[d];
+      acc[d] = T(0);
+    }
+  }
+}
+
 }  // namespace op2b

@@ -171,8 +171,23 @@ struct Held {
   std::vector<op_arg> args;
   bool flux_done = false;  // res_calc: its flux pass already ran (run ahead)
   bool res_zero = false;   // res_calc: res held +0.0 everywhere at the call
+  int part = 0, block = 0;  // OP_part_size and OP_block_size at the call
 };
 std::vector<Held> g_chain;
+
+// the plans of a held res_calc and, when it follows, bres_calc
+ColourKey colour_key(const std::vector<Held> &ch) {
+  ColourKey k;
+  k.rname = ch[0].name.c_str();
+  k.rpart = ch[0].part;
+  k.rblock = ch[0].block;
+  if (ch.size() > 1) {
+    k.bname = ch[1].name.c_str();
+    k.bpart = ch[1].part;
+    k.bblock = ch[1].block;
+  }
+  return k;
+}
 
 bool dat_in(op_dat d, std::initializer_list<op_dat> ds) {
   for (op_dat x : ds)
@@ -220,7 +235,8 @@ bool save_follows_update(const op_arg *u, op_set uset, op_set set, const op_arg 
 bool update_holdable() { return rt().gbl_deferred && rt().reduction == OP2B_REDUCE_TREE; }
 
 bool res_holdable() {
-  return effective_strategy("res_calc") == OP2B_STRATEGY_GATHER && tuning("gather_flux", 1);
+  return effective_strategy("res_calc") == OP2B_STRATEGY_GATHER ? tuning("gather_flux", 1) != 0
+                                                                : coloured_fold();
 }
 
 // ---- loops run ahead of their calls --------------------------------------
@@ -329,7 +345,7 @@ bool run_chain_ahead(const std::vector<Held> &ch) {
   std::vector<GblRequest> held;
   if (!run_res_chain(nullptr, ch[0].set, ch[0].args.data(), ch[1].set, ch[1].args.data(), ua,
                      g_seen_adt.data(), save ? g_seen_save.data() : nullptr, adt_out, save_out,
-                     ch[0].flux_done, &held, ch[0].res_zero))
+                     ch[0].flux_done, &held, ch[0].res_zero, colour_key(ch)))
     return false;
   g_ahead.adt = true;
   g_ahead.save = save;
@@ -396,7 +412,7 @@ void run_chain(const std::vector<Held> &ch, const Held *adt) {
     if (adt && tuning("gather_slots", 1) &&
         run_res_chain(nullptr, ch[0].set, ch[0].args.data(), ch[1].set, ch[1].args.data(),
                       ch[2].args.data(), adt->args.data(), sv.args.data(), nullptr, nullptr,
-                      false, nullptr, ch[0].res_zero))
+                      false, nullptr, ch[0].res_zero, colour_key(ch)))
       return;
     run_chain(std::vector<Held>(ch.begin(), ch.begin() + 3), nullptr);
     run_chain(std::vector<Held>{sv}, adt);
@@ -419,9 +435,9 @@ void run_chain(const std::vector<Held> &ch, const Held *adt) {
         run_res_chain(nullptr, h0.set, a0, h1.set, h1.args.data(), u->args.data(),
                       adt ? adt->args.data() : nullptr, nullptr, nullptr, nullptr,
                       h0.flux_done && h1.kind == K_BRES, nullptr,
-                      h0.kind == K_RES && h0.res_zero))
+                      h0.kind == K_RES && h0.res_zero, colour_key(ch)))
       return;
-    if (!run_res_bres(h0.set, a0, h1.set, h1.args.data())) {
+    if (!run_res_bres(h0.set, a0, h1.set, h1.args.data(), colour_key(ch))) {
       run_kind(h0.kind, 0, h0.name.c_str(), h0.set, a0);
       run_kind(h1.kind, 0, h1.name.c_str(), h1.set, h1.args.data());
     }
@@ -438,6 +454,8 @@ Held make_held(Kind k, char const *name, op_set set, int nargs, const op_arg *ar
   h.kind = k;
   h.name = name;
   h.set = set;
+  h.part = OP_part_size;
+  h.block = OP_block_size;
   h.args.assign(args, args + nargs);
   return h;
 }

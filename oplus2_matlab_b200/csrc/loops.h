@@ -92,11 +92,21 @@ struct ChainArgs {
 };
 bool last_res_chain(ChainArgs *c);
 
+// what a COLOURED res_calc [+ bres_calc] takes its plans from: the loops'
+// names, and OP_part_size and OP_block_size at their calls
+struct ColourKey {
+  char const *rname = "res_calc", *bname = "bres_calc";
+  int rpart = OP_part_size, rblock = OP_block_size, bpart = OP_part_size, bblock = OP_block_size;
+};
+// whether a COLOURED res_calc runs as the flux pass and a fold in the plan's
+// order (knob coloured_fold; 0: a launch per block colour)
+bool coloured_fold();
+
 // fused loop pairs (airfoil.cu); false = not applicable, run them separately
 bool run_save_adt(op_set set, const op_arg *save_args, const op_arg *adt_args);
 bool run_update_adt(op_set set, const op_arg *update_args, const op_arg *adt_args);
 bool run_res_bres(op_set res_set, const op_arg *res_args, op_set bres_set,
-                  const op_arg *bres_args);
+                  const op_arg *bres_args, const ColourKey &key);
 // res_calc, then optionally bres_calc, update and adt_calc (each nullable,
 // in that nesting), through per-cell increment slots; false when the mesh
 // does not suit slots (nothing has run).  save_args: save_soln between
@@ -114,7 +124,8 @@ bool run_res_chain(char const *name, op_set res_set, const op_arg *res_args, op_
                    const op_arg *bres_args, const op_arg *update_args, const op_arg *adt_args,
                    const op_arg *save_args = nullptr, void *adt_out = nullptr,
                    void *save_out = nullptr, bool flux_done = false,
-                   std::vector<GblRequest> *held = nullptr, bool res_zero = false);
+                   std::vector<GblRequest> *held = nullptr, bool res_zero = false,
+                   const ColourKey &key = ColourKey());
 // the flux pass of a res_calc + bres_calc chain before its calls, adt read
 // from adt_now instead of adt's buffer; false when not applicable
 bool run_res_flux_ahead(op_set res_set, const op_arg *res_args, op_set bres_set,

@@ -636,6 +636,7 @@ static void build_plan(DevPlan &p) {
   p.d_ind_offs = (int *)dev_alloc(sizeof(int) * (size_t)nb * (ni ? ni : 1));
   p.d_ind_sizes = (int *)dev_alloc(sizeof(int) * (size_t)nb * (ni ? ni : 1));
   p.d_blkmap = (int *)dev_alloc(sizeof(int) * nb);
+  p.d_blkcol = (int *)dev_alloc(sizeof(int) * nb);
   p.d_ind_maps.assign(ni, nullptr);
   p.d_loc_maps.assign(p.nargs, nullptr);
   for (int a = 0; a < p.nargs; a++)
@@ -716,11 +717,10 @@ static void build_plan(DevPlan &p) {
     iw.wsize[sl] = to_sizes[m];
   }
   unsigned **d_warr = nullptr;
-  int *d_wsz = nullptr, *d_blkcol = nullptr, *d_ncolblk = nullptr, *d_ncolors = nullptr;
+  int *d_wsz = nullptr, *d_ncolblk = nullptr, *d_ncolors = nullptr;
   int nw = (int)warr.size();
   OP2B_CUDA(pool_malloc_async((void **)&d_warr, sizeof(unsigned *) * (nw ? nw : 1), s));
   OP2B_CUDA(pool_malloc_async((void **)&d_wsz, sizeof(int) * (nw ? nw : 1), s));
-  OP2B_CUDA(pool_malloc_async((void **)&d_blkcol, sizeof(int) * nb, s));
   OP2B_CUDA(pool_malloc_async((void **)&d_ncolblk, sizeof(int) * nb, s));
   OP2B_CUDA(pool_malloc_async((void **)&d_ncolors, sizeof(int), s));
   if (nw) {
@@ -728,7 +728,7 @@ static void build_plan(DevPlan &p) {
     OP2B_CUDA(cudaMemcpyAsync(d_wsz, wsz.data(), sizeof(int) * nw, cudaMemcpyHostToDevice, s));
   }
   OP2B_CUDA(cudaMemsetAsync(d_ncolblk, 0, sizeof(int) * nb, s));
-  k_block_colour<<<1, 1024, 0, s>>>(pp, iw, nw, d_warr, d_wsz, d_blkcol, p.d_blkmap, d_ncolblk,
+  k_block_colour<<<1, 1024, 0, s>>>(pp, iw, nw, d_warr, d_wsz, p.d_blkcol, p.d_blkmap, d_ncolblk,
                                     d_ncolors);
 
   // back to the host: the small per-block tables for nshared and the byte
@@ -759,7 +759,6 @@ static void build_plan(DevPlan &p) {
   for (void *w : warr) OP2B_CUDA(cudaFreeAsync(w, s));
   OP2B_CUDA(cudaFreeAsync(d_warr, s));
   OP2B_CUDA(cudaFreeAsync(d_wsz, s));
-  OP2B_CUDA(cudaFreeAsync(d_blkcol, s));
   OP2B_CUDA(cudaFreeAsync(d_ncolblk, s));
   OP2B_CUDA(cudaFreeAsync(d_ncolors, s));
   OP2B_CUDA(cudaFreeAsync(tmp, s));
@@ -1272,6 +1271,61 @@ SlotPlan *get_slot_plan(const GatherPlan *a, const GatherPlan *b) {
   return r->width > 0 ? r : nullptr;
 }
 
+struct ColouredLoop {  // one loop of get_coloured_lists
+  int bsize, nt;
+  const int *blkcol, *thrcol;
+};
+
+// sort a target's entries by what a block kernel does before what else
+__global__ void k_coloured_lists(int ntarget, int W, int na, int nb, const int *__restrict__ ell,
+                                 ColouredLoop A, ColouredLoop B, int *__restrict__ out) {
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ntarget; c += gridDim.x * blockDim.x) {
+    // loop and block colour | strip, thread colour | entry
+    unsigned hi[kMaxSlotWidth];
+    unsigned long long lo[kMaxSlotWidth];
+    int k[kMaxSlotWidth], n = 0;
+    for (int j = 0; j < W; j++) {
+      const int x = ell[(size_t)c * W + j], i = x >> 1;
+      if (i >= na + nb) continue;  // padding
+      const bool b = i >= na;
+      const ColouredLoop &L = b ? B : A;
+      const int e = b ? i - na : i, blk = e / L.bsize;
+      const unsigned h = (b ? 1u << 31 : 0u) | (unsigned)L.blkcol[blk];
+      const unsigned long long l =
+          (unsigned long long)((e - blk * L.bsize) / L.nt) << 32 | (unsigned)L.thrcol[e] << 1 |
+          (x & 1);
+      int m = n++;
+      for (; m > 0 && (hi[m - 1] > h || (hi[m - 1] == h && lo[m - 1] > l)); m--) {
+        hi[m] = hi[m - 1];
+        lo[m] = lo[m - 1];
+        k[m] = k[m - 1];
+      }
+      hi[m] = h;
+      lo[m] = l;
+      k[m] = x;
+    }
+    for (int j = 0; j < W; j++)
+      out[(size_t)c * W + j] =
+          j < n ? (k[j] >> 1) << 2 | (j + 1 == n || hi[j + 1] != hi[j] ? 2 : 0) | (k[j] & 1) : -1;
+  }
+}
+
+const int *get_coloured_lists(SlotPlan *sp, const DevPlan *p, int nt, const DevPlan *pb, int nbt) {
+  for (auto &c : sp->coloured)
+    if (c.p == p && c.pb == pb && c.nt == nt && c.nbt == nbt) return c.d_ell;
+  if ((long long)sp->na + sp->nb + 1 >= (1LL << 29)) return nullptr;
+  SlotPlan::Coloured c{p, pb, nt, nbt, nullptr};
+  c.d_ell = (int *)dev_alloc(sizeof(int) * (size_t)sp->width * sp->ntarget);
+  if (!c.d_ell) return nullptr;
+  const ColouredLoop A{p->bsize, nt, p->d_blkcol, p->d_thrcol};
+  const ColouredLoop B{pb ? pb->bsize : 1, nbt, pb ? pb->d_blkcol : nullptr,
+                       pb ? pb->d_thrcol : nullptr};
+  k_coloured_lists<<<rt().num_sms * 8, 256, 0, rt().stream>>>(sp->ntarget, sp->width, sp->na,
+                                                              sp->nb, sp->d_ell, A, B, c.d_ell);
+  sp->coloured.push_back(c);
+  return c.d_ell;
+}
+
 }  // namespace op2b
 
 using namespace op2b;
@@ -1282,12 +1336,14 @@ void op2b_release_plans() {
     release_tile_plan(up.get());
     dev_free(up->d_ell);
     dev_free(up->d_buf);
+    for (auto &c : up->coloured) dev_free(c.d_ell);
   }
   g_slot_plans.clear();
   for (auto &up : g_plans) {
     DevPlan &p = *up;
     dev_free(p.d_nthrcol); dev_free(p.d_thrcol); dev_free(p.d_offset); dev_free(p.d_nelems);
     dev_free(p.d_ind_offs); dev_free(p.d_ind_sizes); dev_free(p.d_blkmap);
+    dev_free(p.d_blkcol);
     for (int *q : p.d_ind_maps) dev_free(q);
     for (short *q : p.d_loc_maps) dev_free(q);
   }

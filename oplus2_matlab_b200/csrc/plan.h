@@ -25,6 +25,7 @@ struct DevPlan {
   int bsize = 0, nblocks = 0, ncolors = 0, nshared = 0;
   int *d_nthrcol = nullptr, *d_thrcol = nullptr, *d_offset = nullptr, *d_nelems = nullptr;
   int *d_ind_offs = nullptr, *d_ind_sizes = nullptr, *d_blkmap = nullptr;
+  int *d_blkcol = nullptr;  // colour of each block
   std::vector<int *> d_ind_maps;
   std::vector<short *> d_loc_maps;
   std::vector<int> nindirect, ncolblk, colstart;  // host
@@ -91,12 +92,24 @@ struct SlotPlan {
   size_t buf_bytes = 0;
   ChainSched *chain = nullptr;  // built by the first persistent chain launch
   bool chain_unsuited = false;  // a cell tile reads too many flux tiles for it
+  struct Coloured {  // get_coloured_lists
+    const DevPlan *p, *pb;
+    int nt, nbt, *d_ell;
+  };
+  std::vector<Coloured> coloured;
   TilePlan *tile = nullptr;     // built by the first tiled chain launch
   bool tile_unsuited = false;   // no tile size fits shared memory
 };
 // free a slot plan's persistent-chain queue and tile plan (airfoil.cu)
 void release_chain_sched(SlotPlan *sp);
 void release_tile_plan(SlotPlan *sp);
+
+// A slot plan's lists in the order of the two-level colouring of a (plan p, nt
+// threads per block) and b (pb, nbt; nullable): by block colour, then by
+// strip of nt elements of the block, thread colour and slot, b's after a's;
+// entry index << 2 | last of its block << 1 | negate, -1 past the end.
+// Device memory kept with the slot plan; nullptr when the indices do not fit.
+const int *get_coloured_lists(SlotPlan *sp, const DevPlan *p, int nt, const DevPlan *pb, int nbt);
 
 // widest list the fold kernels accept
 constexpr int kMaxSlotWidth = 8;
