@@ -8,8 +8,8 @@
 //    O(N log N) part (gather, sort, dedupe, inverse) runs one CTA per block
 //    and indirect dataset; the thread colouring runs one CTA per block; the
 //    block colouring is the reference's sequential greedy over blocks, run by
-//    one CTA that ORs each block's target masks in parallel.  All of it is
-//    integer work with one exact answer, so the result equals op_plan_core.
+//    one CTA on the blocks' conflicts, which are found in parallel.  All of it
+//    is integer work with one exact answer, so the result equals op_plan_core.
 // 2. A validator for any plan: the reference's op_plan_check
 //    (op_lib_core.c:469-620) plus the colouring checks it leaves out.
 // 3. The owner-computes ("gather") plan used by the GATHER strategy: per
@@ -42,6 +42,8 @@ struct PlanParams {
   int ind_P[kMaxArgs];      // sort size (power of two >= k*bsize)
   int ind_size[kMaxArgs];   // dat bytes per element for ind m
   int ind_dim[kMaxArgs];    // dat dim for ind m
+  int ind_same[kMaxArgs];   // the first ind whose args go through the same maps as m's
+  int arg_same[kMaxArgs];   // the first arg of the same map and index
   int arg_ind[kMaxArgs];    // ind of arg a, or -1
   long long tmp_off[kMaxArgs];
   // OP_INC slots (thread / block colouring): arg and its ind
@@ -83,22 +85,26 @@ __device__ int block_excl_scan(int v, int *total) {
   return excl;
 }
 
+// P a power of two >= 64.  Exchanges over at most 32 places stay inside the 64
+// places of one warp's 32 pairs, so only the wider ones need the CTA's barrier
+// (10 of 55 steps for 1024 values)
 __device__ void bitonic_sort(int *s, int P) {
   for (int k = 2; k <= P; k <<= 1)
     for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = threadIdx.x; i < P; i += blockDim.x) {
-        int ixj = i ^ j;
-        if (ixj > i) {
-          int a = s[i], b = s[ixj];
-          bool up = (i & k) == 0;
-          if ((a > b) == up) {
-            s[i] = b;
-            s[ixj] = a;
-          }
+      for (int t = threadIdx.x; t < P / 2; t += blockDim.x) {
+        const int i = 2 * t - (t & (j - 1));
+        const int a = s[i], b = s[i + j];
+        if ((a > b) == ((i & k) == 0)) {
+          s[i] = b;
+          s[i + j] = a;
         }
       }
-      __syncthreads();
+      // the next step's reach: j / 2, or k after the last step of this k
+      const int reach = j > 1 ? j >> 1 : k;
+      if (j > 32 || reach > 32) __syncthreads();
+      else __syncwarp();
     }
+  __syncthreads();
 }
 
 // one CTA per (block b, indirect dataset m): gather the targets of all args
@@ -111,7 +117,8 @@ __global__ void k_block_unique(PlanParams pp, int *ind_sizes, int *tmp) {
   const int bs = min(pp.bsize, pp.set_size - e0);
   const int k = pp.ind_k[m];
   const int K = k * bs;
-  int P = 1;
+  if (pp.ind_same[m] != m) return;  // computed with that one
+  int P = 64;
   while (P < K) P <<= 1;
   for (int i = threadIdx.x; i < P; i += blockDim.x) {
     int v = INT_MAX;
@@ -133,7 +140,8 @@ __global__ void k_block_unique(PlanParams pp, int *ind_sizes, int *tmp) {
     if (f) out[base + pos] = s[i];
     base += tot;
   }
-  if (threadIdx.x == 0) ind_sizes[m + b * pp.ninds] = base;
+  for (int i = threadIdx.x; i < pp.ninds; i += blockDim.x)
+    if (pp.ind_same[i] == m) ind_sizes[i + b * pp.ninds] = base;
 }
 
 // exclusive scan of ind_sizes over blocks, per indirect dataset
@@ -178,17 +186,21 @@ __global__ void k_block_locmaps(PlanParams pp, IndOut io, const int *ind_sizes,
     io.ind_maps[m][off + u] = t;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < k * bs; i += blockDim.x) {
-    int a = pp.ind_args[pp.ind_first[m] + i / bs];
-    int e = e0 + i % bs;
-    int v = map_at(pp.am, a, e);
-    int lo = 0, hi = nu;  // lower_bound
-    while (lo < hi) {
-      int mid = (lo + hi) >> 1;
-      if (list[mid] < v) lo = mid + 1; else hi = mid;
+  // the local indices of this ind's args, and of the args of later inds that
+  // go through the same maps (their CTAs have none to find)
+  if (pp.ind_same[m] == m)
+    for (int i = threadIdx.x; i < k * bs; i += blockDim.x) {
+      const int j = i / bs;
+      const int e = e0 + i - j * bs;
+      const int v = map_at(pp.am, pp.ind_args[pp.ind_first[m] + j], e);
+      int lo = 0, hi = nu;  // lower_bound
+      while (lo < hi) {
+        int mid = (lo + hi) >> 1;
+        if (list[mid] < v) lo = mid + 1; else hi = mid;
+      }
+      for (int c = m; c < pp.ninds; c++)
+        if (pp.ind_same[c] == m) io.loc_maps[pp.ind_args[pp.ind_first[c] + j]][e] = (short)lo;
     }
-    io.loc_maps[a][e] = (short)lo;
-  }
   // cache lines: element u starts a new line unless its first line is the
   // previous element's last line
   const long long sz = pp.ind_size[m], cls = pp.cls, cls3 = (long long)pp.ind_dim[m] * pp.cls;
@@ -240,9 +252,39 @@ __global__ void k_thread_colour(PlanParams pp, IndOut io, const int *ind_sizes, 
     locs[sl * bs + e] = (unsigned short)io.loc_maps[pp.inc_arg[sl]][e0 + e];
   }
   __syncthreads();
+  for (int i = threadIdx.x; i < pp.mask_words; i += blockDim.x) masks[i] = 0u;
+  for (int e = threadIdx.x; e < bs; e += blockDim.x) col[e] = -1;
+  __syncthreads();
   if (threadIdx.x == 0) {
-    for (int e = 0; e < bs; e++) col[e] = -1;
-    int base = 0, ncol = 0, again = 1;
+    int base = 0, ncol = 0, again = 0;
+    if (pp.ninc == 2) {
+      // the first pass of a loop with two increments, the usual case: the
+      // next element's places are read while this one's masks are on their way
+      unsigned *ma = masks + pp.inc_mbase[0], *mb = masks + pp.inc_mbase[1];
+      const unsigned short *la = locs, *lb = locs + bs;
+      int ia = la[0], ib = lb[0];
+      for (int e = 0; e < bs; e++) {
+        const int i = ia, j = ib;
+        const unsigned xa = ma[i], xb = mb[j];
+        if (e + 1 < bs) {
+          ia = la[e + 1];
+          ib = lb[e + 1];
+        }
+        const int c = __ffs(~(xa | xb)) - 1;
+        if (c < 0) {
+          again = 1;
+          continue;
+        }
+        col[e] = c;
+        ncol = max(ncol, c + 1);
+        ma[i] = xa | 1u << c;
+        if (ma + i == mb + j) continue;  // the same target twice
+        mb[j] = xb | 1u << c;
+      }
+      base = 32;
+    } else {
+      again = 1;
+    }
     while (again) {
       again = 0;
       for (int sl = 0; sl < pp.ninc; sl++) {
@@ -345,6 +387,280 @@ __global__ void k_block_colour(PlanParams pp, IncWork iw, int nwork, unsigned *c
     }
   }
   if (tid == 0) *ncolors_out = ncolors;
+}
+
+// ---- the same colouring from the blocks' conflicts --------------------------
+// A block's colour is the lowest that no earlier block sharing a target with
+// it has (the passes of 32 colours come to the same).  The conflicts are
+// found in parallel -- per target the blocks that increment it, per pair of
+// them a bit in a triangular matrix -- and only the greedy itself goes block
+// after block, over neighbours and colours in shared memory instead of the
+// masks of every target of the block in global memory: 3.4 -> 0.24 ms for
+// 1,586 blocks of 512 edges, 10.6 -> 0.85 ms for 5,620 of 256 (0.15 us a
+// block: a chain of shared loads, a warp reduction and a store), and some
+// 0.06 ms to find the conflicts.
+constexpr int kColourBlocks = 16384;  // blocks the matrix (32 MB) is built for
+constexpr int kColourRow = 64;        // earlier neighbours of a block, for the one-warp greedy
+constexpr int kColourLong = 32;       // blocks of a target paired by one thread
+
+struct ColourSlots {  // the INC arguments; targets of distinct inds apart
+  const int *map[kMaxArgs];
+  int dim[kMaxArgs], idx[kMaxArgs], base[kMaxArgs];
+  int n;
+};
+
+// one (argument, element) after another: its target
+__device__ __forceinline__ int colour_target(const ColourSlots &cs, long long i, int nelem,
+                                             int &e) {
+  const int sl = (int)(i / nelem);
+  e = (int)(i - (long long)sl * nelem);
+  return cs.base[sl] + cs.map[sl][cs.idx[sl] + (size_t)e * cs.dim[sl]];
+}
+
+__global__ void k_colour_count(ColourSlots cs, int nelem, int *cnt) {
+  const long long n = (long long)cs.n * nelem;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x) {
+    int e;
+    atomicAdd(cnt + colour_target(cs, i, nelem, e), 1);
+  }
+}
+
+__global__ void k_colour_scatter(ColourSlots cs, int nelem, int bsize, int *end,
+                                 unsigned short *blocks) {
+  const long long n = (long long)cs.n * nelem;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x) {
+    int e;
+    const int t = colour_target(cs, i, nelem, e);
+    blocks[atomicAdd(end + t, 1)] = (unsigned short)(e / bsize);
+  }
+}
+
+__device__ __forceinline__ void colour_conflict(unsigned *adj, int words, int a, int b) {
+  if (a == b) return;
+  const int hi = max(a, b), lo = min(a, b);
+  unsigned *w = adj + (size_t)hi * words + (lo >> 5);
+  if (*w >> (lo & 31) & 1) return;  // bits are only ever set
+  atomicOr(w, 1u << (lo & 31));
+}
+
+// end[t]: where target t's blocks end, and the next target's begin
+__global__ void k_colour_pairs(int ntarget, const int *end, const unsigned short *blocks,
+                               unsigned *adj, int words, int *long_targets, int *nlong) {
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntarget; t += gridDim.x * blockDim.x) {
+    const int k0 = t ? end[t - 1] : 0, k1 = end[t];
+    if (k1 - k0 > kColourLong) {
+      long_targets[atomicAdd(nlong, 1)] = t;
+      continue;
+    }
+    for (int i = k0 + 1; i < k1; i++)
+      for (int j = k0; j < i; j++) colour_conflict(adj, words, blocks[i], blocks[j]);
+  }
+}
+
+// a target of many blocks: the set of them, then every row of the set
+__global__ void k_colour_long(const int *end, const unsigned short *blocks, unsigned *adj,
+                              int words, int nb, const int *long_targets, const int *nlong) {
+  __shared__ unsigned set[kColourBlocks / 32];
+  for (int l = blockIdx.x; l < *nlong; l += gridDim.x) {
+    const int t = long_targets[l];
+    for (int w = threadIdx.x; w < words; w += blockDim.x) set[w] = 0u;
+    __syncthreads();
+    for (int i = (t ? end[t - 1] : 0) + threadIdx.x; i < end[t]; i += blockDim.x)
+      atomicOr(set + (blocks[i] >> 5), 1u << (blocks[i] & 31));
+    __syncthreads();
+    for (int w = threadIdx.x; w < words; w += blockDim.x) {
+      if (set[w] == 0u) continue;
+      for (int b = w << 5; b < nb; b++) {
+        if (!(set[b >> 5] >> (b & 31) & 1)) continue;
+        const unsigned m = b >> 5 == w ? set[w] & ((1u << (b & 31)) - 1) : set[w];
+        if (m) atomicOr(adj + (size_t)b * words + w, m);
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// each row as a list of its first kColourRow neighbours, one warp per row, and
+// the longest row
+__global__ void k_colour_rows(int nb, int words, const unsigned *adj, unsigned short *list,
+                              int *count, int *longest) {
+  const int lane = threadIdx.x & 31;
+  for (int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < nb;
+       b += (gridDim.x * blockDim.x) >> 5) {
+    int n = 0;
+    for (int w0 = 0; w0 <= b >> 5; w0 += 32) {
+      unsigned bits = w0 + lane <= b >> 5 ? adj[(size_t)b * words + w0 + lane] : 0u;
+      int at = __popc(bits);
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, at, o);
+        if (lane >= o) at += y;
+      }
+      const int all = __shfl_sync(0xffffffffu, at, 31);
+      at += n - __popc(bits);
+      n += all;
+      for (; bits && at < kColourRow; bits &= bits - 1)
+        list[(size_t)b * kColourRow + at++] =
+            (unsigned short)((w0 + lane) * 32 + __ffs(bits) - 1);
+    }
+    if (lane == 0) {
+      count[b] = n;
+      if (n > *longest) atomicMax(longest, n);
+    }
+  }
+}
+
+// blocks grouped by colour, in block order: rank[b] = earlier blocks of its
+// colour.  By all threads of the greedy's CTA; cnt: blocks of each colour
+__device__ void colour_place(int nb, int ncolors, const unsigned short *col, int *cnt,
+                             const unsigned short *rank, int *blk_col, int *blkmap, int *ncolblk,
+                             int *ncolors_out) {
+  const int tid = threadIdx.x;
+  __syncthreads();
+  int run = 0;
+  for (int c0 = 0; c0 < ncolors; c0 += blockDim.x) {
+    const int c = c0 + tid, v = c < ncolors ? cnt[c] : 0;
+    int tot;
+    const int x = block_excl_scan(v, &tot);
+    if (c < ncolors) {
+      ncolblk[c] = v;
+      cnt[c] = run + x;
+    }
+    run += tot;
+  }
+  __syncthreads();
+  for (int b = tid; b < nb; b += blockDim.x) {
+    blk_col[b] = col[b];
+    blkmap[cnt[col[b]] + rank[b]] = b;
+  }
+  if (tid == 0) *ncolors_out = ncolors;
+}
+
+// the greedy when every row fits a list: one warp colours, the CTA brings the
+// next 32 rows
+__global__ void __launch_bounds__(256)
+    k_colour_narrow(int nb, const unsigned short *__restrict__ list, const int *__restrict__ count,
+                    const int *longest, int *blk_col, int *blkmap, int *ncolblk,
+                    int *ncolors_out) {
+  extern __shared__ int colour_smem[];
+  int *cnt = colour_smem;
+  unsigned short *col = (unsigned short *)(cnt + nb), *rank = col + nb;
+  __shared__ unsigned rows[2][32][kColourRow / 2];
+  __shared__ int len[2][32];
+  __shared__ int s_ncolors;
+  if (*longest > kColourRow) return;
+  const int tid = threadIdx.x, lane = tid & 31;
+  auto stage = [&](int b0, int buf, int first) {  // by the threads from `first` on
+    for (int i = tid - first; i < 32 * (kColourRow / 2); i += 256 - first) {
+      const int r = i / (kColourRow / 2), k = i % (kColourRow / 2);
+      if (b0 + r < nb)
+        rows[buf][r][k] =
+            __ldg(reinterpret_cast<const unsigned *>(list + (size_t)(b0 + r) * kColourRow) + k);
+    }
+    if (tid >= first && tid < first + 32)
+      len[buf][tid - first] = b0 + tid - first < nb ? __ldg(count + b0 + tid - first) : 0;
+  };
+  for (int b = tid; b < nb; b += 256) cnt[b] = 0;
+  stage(0, 0, 0);
+  int ncolors = 0;
+  for (int b0 = 0, buf = 0; b0 < nb; b0 += 32, buf ^= 1) {
+    __syncthreads();
+    if (tid >= 32) {
+      if (b0 + 32 < nb) stage(b0 + 32, buf ^ 1, 32);
+      continue;
+    }
+    // a row's neighbours and their colours are read while the row before it
+    // is coloured; that row's own colour is put in by hand
+    const int nr = min(32, nb - b0);
+    int ia, ib, ca, cb, mine = 0;
+    auto read = [&](int r) {
+      const unsigned pair = rows[buf][r][lane];  // neighbours 2 lane and 2 lane + 1
+      const int n = len[buf][r];
+      ia = 2 * lane < n ? (int)(pair & 0xffffu) : -1;
+      ib = 2 * lane + 1 < n ? (int)(pair >> 16) : -1;
+      ca = ia >= 0 ? (int)col[ia] : -1;
+      cb = ib >= 0 ? (int)col[ib] : -1;
+    };
+    read(0);
+    for (int r = 0; r < nr; r++) {
+      const int b = b0 + r, xa = ca, xb = cb;
+      if (r + 1 < nr) read(r + 1);
+      int c = 0;
+      for (int base = 0;; base += 32) {
+        unsigned mask = 0;
+        if (xa >= base && xa < base + 32) mask |= 1u << (xa - base);
+        if (xb >= base && xb < base + 32) mask |= 1u << (xb - base);
+        mask = __reduce_or_sync(0xffffffffu, mask);
+        if (mask != ~0u) {
+          c = base + __ffs(~mask) - 1;
+          break;
+        }
+      }
+      if (lane == 0) col[b] = (unsigned short)c;
+      __syncwarp();
+      if (ia == b) ca = c;
+      if (ib == b) cb = c;
+      if (lane == r) mine = c;
+      ncolors = max(ncolors, c + 1);
+    }
+    // ranks of the 32 blocks among those of their colour
+    const unsigned same = __match_any_sync(0xffffffffu, lane < nr ? mine : -1 - lane);
+    const unsigned before = same & ((1u << lane) - 1);
+    if (lane < nr) rank[b0 + lane] = (unsigned short)(cnt[mine] + __popc(before));
+    __syncwarp();
+    if (lane < nr && before == 0) cnt[mine] += __popc(same);
+    __syncwarp();
+  }
+  if (tid == 0) s_ncolors = ncolors;
+  __syncthreads();
+  colour_place(nb, s_ncolors, col, cnt, rank, blk_col, blkmap, ncolblk, ncolors_out);
+}
+
+// the greedy for wide rows (a numbering without locality): all threads read a
+// row, half a word each; seen[c] = the last block that has a neighbour of
+// colour c
+__global__ void __launch_bounds__(1024)
+    k_colour_wide(int nb, int words, const unsigned *__restrict__ adj, const int *longest,
+                  int *blk_col, int *blkmap, int *ncolblk, int *ncolors_out) {
+  extern __shared__ int colour_smem[];
+  int *cnt = colour_smem, *seen = cnt + nb;
+  unsigned short *col = (unsigned short *)(seen + nb + 1), *rank = col + nb;
+  __shared__ int s_first[2];
+  if (*longest <= kColourRow) return;
+  const int tid = threadIdx.x, halves = 2 * words;  // at most 1024
+  for (int b = tid; b < nb; b += 1024) cnt[b] = 0;
+  for (int b = tid; b <= nb; b += 1024) seen[b] = -1;
+  if (tid < 2) s_first[tid] = nb;
+  int ncolors = 0;
+  unsigned next = tid < halves ? __ldg(adj + (tid >> 1)) : 0u;
+  __syncthreads();
+  for (int b = 0; b < nb; b++) {
+    unsigned bits = next >> (16 * (tid & 1)) & 0xffffu;
+    if (b + 1 < nb && tid < halves) next = __ldg(adj + (size_t)(b + 1) * words + (tid >> 1));
+    while (bits) {
+      const int j = tid * 16 + __ffs(bits) - 1;
+      bits &= bits - 1;
+      seen[col[j]] = b;
+    }
+    __syncthreads();
+    // the first colour not seen; ncolors itself never is
+    for (int c0 = 0; c0 <= ncolors; c0 += 1024) {
+      const bool free_c = c0 + tid <= ncolors && seen[c0 + tid] != b;
+      const unsigned m = __ballot_sync(0xffffffffu, free_c);
+      if (m && (tid & 31) == 0) atomicMin(&s_first[b & 1], c0 + tid + __ffs(m) - 1);
+    }
+    __syncthreads();
+    const int c = s_first[b & 1];
+    ncolors = max(ncolors, c + 1);
+    if (tid == 0) {
+      col[b] = (unsigned short)c;
+      rank[b] = (unsigned short)cnt[c]++;
+      s_first[(b & 1) ^ 1] = nb;
+    }
+    __syncthreads();
+  }
+  colour_place(nb, ncolors, col, cnt, rank, blk_col, blkmap, ncolblk, ncolors_out);
 }
 
 // ----------------------------------------------------------- validation --
@@ -551,9 +867,28 @@ static bool fill_params(PlanParams &pp, const DevPlan &p, std::vector<int> &to_s
   for (int m = 0; m < p.ninds; m++) {
     pp.tmp_off[m] = off;
     off += (long long)pp.ind_k[m] * p.bsize * p.nblocks;
-    int P = 1;
+    int P = 64;
     while (P < pp.ind_k[m] * p.bsize) P <<= 1;
     pp.ind_P[m] = P;
+  }
+  // q, adt and res of airfoil's res_calc all go through pecell: their distinct
+  // targets and local indices are found once
+  for (int a = 0; a < p.nargs; a++) {
+    pp.arg_same[a] = a;
+    for (int c = 0; c < a && pp.arg_same[a] == a; c++)
+      if (p.inds[a] >= 0 && p.inds[c] >= 0 && p.maps[c] == p.maps[a] && p.idxs[c] == p.idxs[a])
+        pp.arg_same[a] = c;
+  }
+  for (int m = 0; m < p.ninds; m++) {
+    pp.ind_same[m] = m;
+    for (int c = 0; c < m && pp.ind_same[m] == m; c++) {
+      bool same = pp.ind_k[c] == pp.ind_k[m];
+      for (int i = 0; i < pp.ind_k[m] && same; i++)
+        same = pp.arg_same[pp.ind_args[pp.ind_first[c] + i]] ==
+               pp.arg_same[pp.ind_args[pp.ind_first[m] + i]];
+      if (same) pp.ind_same[m] = c;
+    }
+    pp.tmp_off[m] = pp.tmp_off[pp.ind_same[m]];
   }
   // INC slots and their mask areas (one area per distinct ind)
   int mbase_of_ind[kMaxArgs];
@@ -593,6 +928,106 @@ static size_t allow_smem(K kernel) {
   size_t dyn = smem_optin() - fa.sharedSizeBytes;
   OP2B_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
   return dyn;
+}
+
+// block colours, blkmap and the blocks per colour from the conflicts of the
+// blocks; false for more blocks (or targets) than that is built for
+static bool colour_blocks(const DevPlan &p, const PlanParams &pp, const std::vector<int> &to_sizes,
+                          int *d_ncolblk, int *d_ncolors, cudaStream_t s) {
+  const int nb = p.nblocks, n = p.set->size, words = (nb + 31) / 32;
+  if (nb > kColourBlocks) return false;
+  ColourSlots cs;
+  memset(&cs, 0, sizeof cs);
+  long long nt = 0;
+  std::vector<int> base(kMaxArgs, -1);
+  for (int sl = 0; sl < pp.ninc; sl++) {
+    const int m = pp.inc_ind[sl], a = pp.inc_arg[sl];
+    if (base[m] < 0) {
+      base[m] = (int)nt;
+      nt += to_sizes[m];
+    }
+    cs.map[sl] = pp.am.map[a];
+    cs.dim[sl] = pp.am.dim[a];
+    cs.idx[sl] = pp.am.idx[a];
+    cs.base[sl] = base[m];
+    cs.n = sl + 1;
+  }
+  const long long nent = (long long)pp.ninc * n;
+  if (nt >= (1LL << 31) - 1 || nent >= (1LL << 31) - 1) return false;
+  // adjacency | longest row, number of long targets | per target: blocks' end
+  // | long targets | row lengths | rows | blocks
+  const size_t adj_bytes = sizeof(unsigned) * (size_t)nb * words;
+  const size_t ntz = (size_t)std::max(1LL, nt);
+  char *mem = nullptr;
+  const size_t bytes =
+      adj_bytes + sizeof(int) * (2 + 2 * ntz + nb) +
+      sizeof(unsigned short) * ((size_t)nb * kColourRow + (size_t)std::max(1LL, nent));
+  if (pool_malloc_async((void **)&mem, bytes, s) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  unsigned *adj = (unsigned *)mem;
+  int *longest = (int *)(mem + adj_bytes), *nlong = longest + 1, *end = longest + 2;
+  int *longs = end + ntz, *count = longs + ntz;
+  unsigned short *list = (unsigned short *)(count + nb), *blocks = list + (size_t)nb * kColourRow;
+  OP2B_CUDA(cudaMemsetAsync(mem, 0, adj_bytes + 2 * sizeof(int) + sizeof(int) * ntz, s));
+  if (pp.ninc) {
+    const int grid = rt().num_sms * 8;
+    k_colour_count<<<grid, 256, 0, s>>>(cs, n, end);
+    exclusive_scan_nosync(end, end, (int)nt, s);
+    k_colour_scatter<<<grid, 256, 0, s>>>(cs, n, p.bsize, end, blocks);
+    k_colour_pairs<<<grid, 256, 0, s>>>((int)nt, end, blocks, adj, words, longs, nlong);
+    k_colour_long<<<rt().num_sms, 256, 0, s>>>(end, blocks, adj, words, nb, longs, nlong);
+  }
+  k_colour_rows<<<std::min(rt().num_sms * 8, (nb + 7) / 8), 256, 0, s>>>(nb, words, adj, list,
+                                                                        count, longest);
+  allow_smem(k_colour_narrow);
+  allow_smem(k_colour_wide);
+  k_colour_narrow<<<1, 256, 8 * (size_t)nb, s>>>(nb, list, count, longest, p.d_blkcol,
+                                                 p.d_blkmap, d_ncolblk, d_ncolors);
+  k_colour_wide<<<1, 1024, 12 * (size_t)nb + 4, s>>>(nb, words, adj, longest, p.d_blkcol,
+                                                     p.d_blkmap, d_ncolblk, d_ncolors);
+  OP2B_CUDA(cudaFreeAsync(mem, s));
+  return true;
+}
+
+// the same for any number of blocks: a block's colour from the masks of its
+// targets, one block after another
+static void colour_blocks_by_targets(const DevPlan &p, const PlanParams &pp,
+                                     const std::vector<int> &to_sizes, int *d_ncolblk,
+                                     int *d_ncolors, cudaStream_t s) {
+  IncWork iw;  // one mask array per distinct INC ind
+  memset(&iw, 0, sizeof iw);
+  std::vector<unsigned *> warr;
+  std::vector<int> wsz;
+  std::vector<int> ind_w(kMaxArgs, -1);
+  for (int sl = 0; sl < pp.ninc; sl++) {
+    int m = pp.inc_ind[sl];
+    if (ind_w[m] < 0) {
+      unsigned *w = nullptr;
+      OP2B_CUDA(pool_malloc_async((void **)&w, sizeof(unsigned) * (size_t)to_sizes[m], s));
+      ind_w[m] = (int)warr.size();
+      warr.push_back(w);
+      wsz.push_back(to_sizes[m]);
+    }
+    iw.work[sl] = warr[ind_w[m]];
+    iw.wsize[sl] = to_sizes[m];
+  }
+  unsigned **d_warr = nullptr;
+  int *d_wsz = nullptr;
+  int nw = (int)warr.size();
+  OP2B_CUDA(pool_malloc_async((void **)&d_warr, sizeof(unsigned *) * (nw ? nw : 1), s));
+  OP2B_CUDA(pool_malloc_async((void **)&d_wsz, sizeof(int) * (nw ? nw : 1), s));
+  if (nw) {
+    OP2B_CUDA(cudaMemcpyAsync(d_warr, warr.data(), sizeof(unsigned *) * nw, cudaMemcpyHostToDevice, s));
+    OP2B_CUDA(cudaMemcpyAsync(d_wsz, wsz.data(), sizeof(int) * nw, cudaMemcpyHostToDevice, s));
+  }
+  k_block_colour<<<1, 1024, 0, s>>>(pp, iw, nw, d_warr, d_wsz, p.d_blkcol, p.d_blkmap, d_ncolblk,
+                                    d_ncolors);
+  OP2B_CUDA(cudaStreamSynchronize(s));  // the host tables have been read
+  for (void *w : warr) OP2B_CUDA(cudaFreeAsync(w, s));
+  OP2B_CUDA(cudaFreeAsync(d_warr, s));
+  OP2B_CUDA(cudaFreeAsync(d_wsz, s));
 }
 
 static void build_plan(DevPlan &p) {
@@ -670,7 +1105,8 @@ static void build_plan(DevPlan &p) {
     for (int m = 0; m < ni; m++) maxP = std::max(maxP, pp.ind_P[m]);
     size_t sm = sizeof(int) * (size_t)maxP;
     allow_smem(k_block_unique);
-    k_block_unique<<<dim3(nb, ni), 1024, sm, s>>>(pp, p.d_ind_sizes, tmp);
+    k_block_unique<<<dim3(nb, ni), std::min(1024, std::max(32, maxP / 2)), sm, s>>>(
+        pp, p.d_ind_sizes, tmp);
     k_scan_blocks<<<ni, 1024, 0, s>>>(nb, ni, p.d_ind_sizes, p.d_ind_offs, d_nind);
     OP2B_CUDA(cudaMemcpyAsync(p.nindirect.data(), d_nind, sizeof(int) * ni,
                               cudaMemcpyDeviceToHost, s));
@@ -698,38 +1134,12 @@ static void build_plan(DevPlan &p) {
   allow_smem(k_thread_colour);
   k_thread_colour<<<nb, 128, sm3, s>>>(pp, io, p.d_ind_sizes, p.d_thrcol, p.d_nthrcol);
 
-  // block colouring: one mask array per distinct INC ind
-  IncWork iw;
-  memset(&iw, 0, sizeof iw);
-  std::vector<unsigned *> warr;
-  std::vector<int> wsz;
-  std::vector<int> ind_w(kMaxArgs, -1);
-  for (int sl = 0; sl < pp.ninc; sl++) {
-    int m = pp.inc_ind[sl];
-    if (ind_w[m] < 0) {
-      unsigned *w = nullptr;
-      OP2B_CUDA(pool_malloc_async((void **)&w, sizeof(unsigned) * (size_t)to_sizes[m], s));
-      ind_w[m] = (int)warr.size();
-      warr.push_back(w);
-      wsz.push_back(to_sizes[m]);
-    }
-    iw.work[sl] = warr[ind_w[m]];
-    iw.wsize[sl] = to_sizes[m];
-  }
-  unsigned **d_warr = nullptr;
-  int *d_wsz = nullptr, *d_ncolblk = nullptr, *d_ncolors = nullptr;
-  int nw = (int)warr.size();
-  OP2B_CUDA(pool_malloc_async((void **)&d_warr, sizeof(unsigned *) * (nw ? nw : 1), s));
-  OP2B_CUDA(pool_malloc_async((void **)&d_wsz, sizeof(int) * (nw ? nw : 1), s));
+  int *d_ncolblk = nullptr, *d_ncolors = nullptr;
   OP2B_CUDA(pool_malloc_async((void **)&d_ncolblk, sizeof(int) * nb, s));
   OP2B_CUDA(pool_malloc_async((void **)&d_ncolors, sizeof(int), s));
-  if (nw) {
-    OP2B_CUDA(cudaMemcpyAsync(d_warr, warr.data(), sizeof(unsigned *) * nw, cudaMemcpyHostToDevice, s));
-    OP2B_CUDA(cudaMemcpyAsync(d_wsz, wsz.data(), sizeof(int) * nw, cudaMemcpyHostToDevice, s));
-  }
   OP2B_CUDA(cudaMemsetAsync(d_ncolblk, 0, sizeof(int) * nb, s));
-  k_block_colour<<<1, 1024, 0, s>>>(pp, iw, nw, d_warr, d_wsz, p.d_blkcol, p.d_blkmap, d_ncolblk,
-                                    d_ncolors);
+  if (!colour_blocks(p, pp, to_sizes, d_ncolblk, d_ncolors, s))
+    colour_blocks_by_targets(p, pp, to_sizes, d_ncolblk, d_ncolors, s);
 
   // back to the host: the small per-block tables for nshared and the byte
   // models, the colour counts for the launch loop
@@ -756,9 +1166,6 @@ static void build_plan(DevPlan &p) {
   p.colstart.assign(ncolors + 1, 0);
   for (int c = 0; c < ncolors; c++) p.colstart[c + 1] = p.colstart[c] + p.ncolblk[c];
 
-  for (void *w : warr) OP2B_CUDA(cudaFreeAsync(w, s));
-  OP2B_CUDA(cudaFreeAsync(d_warr, s));
-  OP2B_CUDA(cudaFreeAsync(d_wsz, s));
   OP2B_CUDA(cudaFreeAsync(d_ncolblk, s));
   OP2B_CUDA(cudaFreeAsync(d_ncolors, s));
   OP2B_CUDA(cudaFreeAsync(tmp, s));
