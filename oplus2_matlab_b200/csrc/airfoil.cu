@@ -44,7 +44,7 @@ __device__ __forceinline__ int at(const IdxMap &m, int e) {
 // idx 0 and 1 (pedge, pecell, pbedge) this is a single 8-byte load.
 __device__ __forceinline__ void at2(const IdxMap &a, const IdxMap &b, int e, int &i, int &j) {
   if (a.map && a.map == b.map && a.dim == 2 && a.idx == 0 && b.idx == 1) {
-    int2 v = __ldg(reinterpret_cast<const int2 *>(a.map) + e);
+    int2 v = ld_stream(reinterpret_cast<const int2 *>(a.map) + e);
     i = v.x;
     j = v.y;
   } else {
@@ -91,7 +91,7 @@ __global__ void k_adt_calc(int n, IdxMap m0, IdxMap m1, IdxMap m2, IdxMap m3, Id
       const int c = base + u * stride;
       if (c >= n) continue;
       if (quad) {
-        int4 v = __ldg(reinterpret_cast<const int4 *>(m0.map) + c);
+        int4 v = ld_stream(reinterpret_cast<const int4 *>(m0.map) + c);
         nd[u][0] = v.x; nd[u][1] = v.y; nd[u][2] = v.z; nd[u][3] = v.w;
       } else {
         nd[u][0] = at(m0, c); nd[u][1] = at(m1, c); nd[u][2] = at(m2, c); nd[u][3] = at(m3, c);
@@ -422,8 +422,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 4)
   const unsigned stride = gridDim.x * blockDim.x;
   int2 nn = make_int2(0, 0), cc = make_int2(0, 0);
   if (i0 < n_e) {  // map entries: read-only, fetched before the wait
-    nn = __ldg(pedge + i0);
-    cc = __ldg(pecell + i0);
+    nn = ld_stream(pedge + i0);
+    cc = ld_stream(pecell + i0);
   }
   pdl_wait();
   pdl_trigger();
@@ -437,8 +437,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 4)
       ld2(x + 2u * (unsigned)nn.y, s);
       const T d1 = __ldg(adt + (unsigned)cc.x), d2 = __ldg(adt + (unsigned)cc.y);
       if (i + stride < n_e) {
-        nn = __ldg(pedge + i + stride);
-        cc = __ldg(pecell + i + stride);
+        nn = ld_stream(pedge + i + stride);
+        cc = ld_stream(pecell + i + stride);
       }
       res_flux(p, s, q1, q2, d1, d2, K.gm1, K.eps, f);
     } else {
@@ -464,7 +464,7 @@ __device__ __forceinline__ void fold_list(const int *__restrict__ ell, int W,
   for (int j0 = 0; j0 < W; j0 += 4) {
     int k[4];
     if (W - j0 >= 4 && ((W & 3) == 0)) {
-      const int4 kk = __ldg(reinterpret_cast<const int4 *>(ell + (size_t)c * W + j0));
+      const int4 kk = ld_stream(reinterpret_cast<const int4 *>(ell + (size_t)c * W + j0));
       k[0] = kk.x; k[1] = kk.y; k[2] = kk.z; k[3] = kk.w;
     } else {
 #pragma unroll
@@ -536,7 +536,7 @@ __global__ void __launch_bounds__(256, MINB)
       list_head(ell, W, c, kk[u]);
       if (ADT) {
         if (quad) {
-          int4 v = __ldg(reinterpret_cast<const int4 *>(N.m0.map) + c);
+          int4 v = ld_stream(reinterpret_cast<const int4 *>(N.m0.map) + c);
           nn[u][0] = v.x; nn[u][1] = v.y; nn[u][2] = v.z; nn[u][3] = v.w;
         } else {
           nn[u][0] = at(N.m0, c); nn[u][1] = at(N.m1, c);
@@ -657,7 +657,7 @@ __global__ void __launch_bounds__(256, MINB)
     list_head(ell, W, c, kk);
     if (ADT) {
       if (quad) {
-        int4 v = __ldg(reinterpret_cast<const int4 *>(N.m0.map) + c);
+        int4 v = ld_stream(reinterpret_cast<const int4 *>(N.m0.map) + c);
         nn[0] = v.x; nn[1] = v.y; nn[2] = v.z; nn[3] = v.w;
       } else {
         nn[0] = at(N.m0, c); nn[1] = at(N.m1, c); nn[2] = at(N.m2, c); nn[3] = at(N.m3, c);
@@ -885,7 +885,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2)
         list_head(ell, W, c, k);
         int nd[4] = {0, 0, 0, 0};
         if (ADT) {
-          const int4 v = __ldg(reinterpret_cast<const int4 *>(N.m0.map) + c);
+          const int4 v = ld_stream(reinterpret_cast<const int4 *>(N.m0.map) + c);
           nd[0] = v.x; nd[1] = v.y; nd[2] = v.z; nd[3] = v.w;
         }
         T r[4], qo[4], f[4][4], xs[4][2];
@@ -1459,7 +1459,7 @@ __global__ void k_save_adt(int n, const T *__restrict__ q, T *__restrict__ qold,
   int nd[4];
   auto nodes = [&](int c) {
     if (quad) {
-      int4 v = __ldg(reinterpret_cast<const int4 *>(m0.map) + c);
+      int4 v = ld_stream(reinterpret_cast<const int4 *>(m0.map) + c);
       nd[0] = v.x; nd[1] = v.y; nd[2] = v.z; nd[3] = v.w;
     } else {
       nd[0] = at(m0, c); nd[1] = at(m1, c); nd[2] = at(m2, c); nd[3] = at(m3, c);
@@ -1500,7 +1500,7 @@ __global__ void k_update_adt(int n, const T *__restrict__ qold, T *__restrict__ 
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
     int nd[4];
     if (quad) {
-      int4 v = __ldg(reinterpret_cast<const int4 *>(m0.map) + c);
+      int4 v = ld_stream(reinterpret_cast<const int4 *>(m0.map) + c);
       nd[0] = v.x; nd[1] = v.y; nd[2] = v.z; nd[3] = v.w;
     } else {
       nd[0] = at(m0, c); nd[1] = at(m1, c); nd[2] = at(m2, c); nd[3] = at(m3, c);

@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 6 : 4)
   const SolveDev<T> *d = sd + t.solve;
   const int4 *pcell = reinterpret_cast<const int4 *>(d->pcell);
   int4 nd = make_int4(0, 0, 0, 0);
-  if ((int)threadIdx.x < t.count) nd = __ldg(pcell + t.start + threadIdx.x);  // read-only
+  if ((int)threadIdx.x < t.count) nd = ld_stream(pcell + t.start + threadIdx.x);  // read-only
   pdl_wait();
   pdl_trigger();
   if (!solve_active(st, t.solve)) return;
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 6 : 4)
     ld2(x + 2 * (size_t)nd.y, b);
     ld2(x + 2 * (size_t)nd.z, e);
     ld2(x + 2 * (size_t)nd.w, f);
-    if (i + kThreads < t.count) nd = __ldg(pcell + c + kThreads);
+    if (i + kThreads < t.count) nd = ld_stream(pcell + c + kThreads);
     st4(qold + 4 * (size_t)c, qq);
     adt[c] = adt_calc(a, b, e, f, qq, K);
   }
@@ -168,8 +168,8 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 8 : 4)
   const int i0 = t.start + threadIdx.x, end = t.start + t.count;
   int2 nn = make_int2(0, 0), cc = make_int2(0, 0);
   if (i0 < end && i0 < ne) {  // map entries: read-only
-    nn = __ldg(pedge + i0);
-    cc = __ldg(pecell + i0);
+    nn = ld_stream(pedge + i0);
+    cc = ld_stream(pecell + i0);
   }
   pdl_wait();
   pdl_trigger();
@@ -181,8 +181,8 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 8 : 4)
     T f[4];
     if (i < ne) {
       if (i != i0) {
-        nn = __ldg(pedge + i);
-        cc = __ldg(pecell + i);
+        nn = ld_stream(pedge + i);
+        cc = ld_stream(pecell + i);
       }
       T p[2], s[2], q1[4], q2[4];
       ld4(q + 4 * (size_t)cc.x, q1);
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? (MODE == 1 ? 4 : 3)
   int4 nd = make_int4(0, 0, 0, 0);
   if ((int)threadIdx.x < t.count) {
     list_head(ell, W, t.start + threadIdx.x, k);
-    if (ADT) nd = __ldg(pcell + t.start + threadIdx.x);
+    if (ADT) nd = ld_stream(pcell + t.start + threadIdx.x);
   }
   pdl_wait();
   pdl_trigger();
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? (MODE == 1 ? 4 : 3)
     int kc[4] = {k[0], k[1], k[2], k[3]};
     if (i + kThreads < t.count) {
       list_head(ell, W, c + kThreads, k);
-      if (ADT) nd = __ldg(pcell + c + kThreads);
+      if (ADT) nd = ld_stream(pcell + c + kThreads);
     }
 #pragma unroll
     for (int m = 0; m < 4; m++) add_listed(r, kc[m], f[m]);
