@@ -416,10 +416,21 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 4)
     k_res_flux_pair(int ne, const int2 *__restrict__ pedge, const int2 *__restrict__ pecell,
                     const T *__restrict__ x, const T *__restrict__ q,
                     const T *__restrict__ adt, BresEdges<T> B, T *__restrict__ v,
-                    AirConsts<T> K) {
+                    AirConsts<T> K, RedTail<T> tail) {
   const unsigned total = (unsigned)ne + (unsigned)B.n, n_e = (unsigned)ne;
-  const unsigned i0 = blockIdx.x * blockDim.x + threadIdx.x;
-  const unsigned stride = gridDim.x * blockDim.x;
+  unsigned cta = blockIdx.x, ctas = gridDim.x;
+  if (tail.n) {  // one more CTA, for what the kernel before left to fold
+    if (cta == 0) {
+      pdl_wait();
+      pdl_trigger();
+      red_tail_fold(tail);
+      return;
+    }
+    cta--;
+    ctas--;
+  }
+  const unsigned i0 = cta * blockDim.x + threadIdx.x;
+  const unsigned stride = ctas * blockDim.x;
   int2 nn = make_int2(0, 0), cc = make_int2(0, 0);
   if (i0 < n_e) {  // map entries: read-only, fetched before the wait
     nn = ld_stream(pedge + i0);
@@ -629,6 +640,115 @@ __global__ void __launch_bounds__(256, MINB)
       }
   }
   if (seq) return;
+  const T v[1] = {rms}, id[1] = {T(0)};
+  RedSlot<T> sl[1] = {slot};
+  grid_finish<T, OpSum, OpSum, 1>(v, id, OpSum(), OpSum(), sl, ticket);
+}
+
+// The same pass for the airfoil shape: lists of four, adt_calc's x through one
+// dim-4 map in order and of one dataset, indices that fit 32 bits.  Every
+// load of a thread's next cell -- its own streams, its nodes and its listed
+// values -- is issued before this cell's arithmetic, and the indices two cells
+// ahead, so a warp has a cell's loads in flight while it computes.
+template <class T>
+struct CellIn {
+  T f[4][4], x[4][2], qo[4], r[4], ad;
+};
+constexpr int kFoldThreads = 256;
+template <class T, bool ADT, bool SAVE, bool NORES, bool COL>
+__global__ void __launch_bounds__(kFoldThreads, sizeof(T) == 4 ? 2 : 1)
+    k_fold_cells(unsigned n, const int4 *__restrict__ ell, const T *__restrict__ vals,
+                 const T *qold, T *q, T *res, const T *adt, const int4 *__restrict__ pcell,
+                 const T *__restrict__ x, AirConsts<T> K, T *seq, RedSlot<T> slot,
+                 unsigned *ticket, T *qsave, T *adt_out) {
+  const unsigned stride = gridDim.x * blockDim.x;
+  unsigned c = blockIdx.x * blockDim.x + threadIdx.x;
+  T rms = T(0);
+  auto index = [&](unsigned c, int4 &k, int4 &nd) {
+    k = ld_stream(ell + c);
+    if (ADT) nd = ld_stream(pcell + c);
+  };
+  auto own = [&](unsigned c, const int4 &nd, CellIn<T> &d) {
+    if (!NORES) ldw4(res + 4u * c, d.r);
+    ldw4(qold + 4u * c, d.qo);
+    d.ad = adt[c];
+    if (ADT) {
+      ld2(x + 2u * (unsigned)nd.x, d.x[0]);
+      ld2(x + 2u * (unsigned)nd.y, d.x[1]);
+      ld2(x + 2u * (unsigned)nd.z, d.x[2]);
+      ld2(x + 2u * (unsigned)nd.w, d.x[3]);
+    }
+  };
+  auto listed = [&](const int4 &k, CellIn<T> &d) {
+    constexpr int S = COL ? 2 : 1;
+    if (!COL || k.x >= 0) ld4(vals + 4u * (unsigned)(k.x >> S), d.f[0]);
+    if (!COL || k.y >= 0) ld4(vals + 4u * (unsigned)(k.y >> S), d.f[1]);
+    if (!COL || k.z >= 0) ld4(vals + 4u * (unsigned)(k.z >> S), d.f[2]);
+    if (!COL || k.w >= 0) ld4(vals + 4u * (unsigned)(k.w >> S), d.f[3]);
+  };
+  auto cell = [&](unsigned c, const int4 &k4, const CellIn<T> &d) {
+    const int k[4] = {k4.x, k4.y, k4.z, k4.w};
+    T r[4], acc[4] = {T(0), T(0), T(0), T(0)};
+#pragma unroll
+    for (int i = 0; i < 4; i++) r[i] = NORES ? T(0) : d.r[i];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      if (COL) add_coloured(r, acc, k[j], d.f[j]);
+      else add_signed(r, k[j], d.f[j]);
+    }
+    // airfoil/update.h:1-12
+    const T adti = rcp(d.ad);
+    T qn[4], sq[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const T del = adti * r[i];
+      qn[i] = d.qo[i] - del;
+      sq[i] = del * del;
+      rms += sq[i];
+    }
+    st4(q + 4u * c, qn);
+    if (SAVE) st4(qsave + 4u * c, qn);  // airfoil/save_soln.h:1-3
+    const T z[4] = {T(0), T(0), T(0), T(0)};
+    if (!NORES) st4(res + 4u * c, z);
+    if (seq) st4(seq + 4 * (size_t)c, sq);
+    if (ADT) adt_out[c] = adt_calc(d.x[0], d.x[1], d.x[2], d.x[3], qn, K);
+  };
+  int4 ka = make_int4(0, 0, 0, 0), na = ka, kb = ka, nb = ka;
+  CellIn<T> da, db;
+  // before the previous kernel has finished: see k_fold_update
+  if (c < n) {
+    index(c, ka, na);
+    own(c, na, da);
+  }
+  if (c + stride < n) index(c + stride, kb, nb);
+  pdl_wait();
+  pdl_trigger();
+  if (c < n) listed(ka, da);
+  auto step = [&](const int4 &k, const CellIn<T> &d, int4 &kn, int4 &nn, CellIn<T> &dn) {
+    const unsigned c1 = c + stride, c2 = c1 + stride;
+    const int4 know = k, knext = kn;
+    if (c1 < n) {
+      own(c1, nn, dn);
+      listed(kn, dn);
+    }
+    if (c2 < n) index(c2, kn, nn);
+    cell(c, know, d);
+    return knext;
+  };
+  for (; c < n;) {
+    ka = step(ka, da, kb, nb, db);
+    c += stride;
+    if (c >= n) break;
+    ka = step(ka, db, kb, nb, da);
+    c += stride;
+  }
+  if (seq) return;
+  if (!ticket) {  // the next kernel folds the partials
+    __shared__ T ws[32];
+    rms = block_fold(rms, T(0), OpSum(), ws);
+    if (threadIdx.x == 0) slot.partials[blockIdx.x] = rms;
+    return;
+  }
   const T v[1] = {rms}, id[1] = {T(0)};
   RedSlot<T> sl[1] = {slot};
   grid_finish<T, OpSum, OpSum, 1>(v, id, OpSum(), OpSum(), sl, ticket);
@@ -1732,10 +1852,13 @@ static void launch_flux(const op_arg *ra, const ResEdges<T> &E, const BresEdges<
                      ra[4].dat == ra[5].dat && (long long)nval < (1LL << 30) &&
                      (long long)ra[2].dat->set->size < (1LL << 30) &&
                      (long long)ra[0].dat->set->size < (1LL << 30);
-  if (shape && tuning("flux_pair", 1))
-    launch_pdl(k_res_flux_pair<T>, fgrid, 256, 0, s, E.n,
+  if (shape && tuning("flux_pair", 1)) {
+    const RedTail<T> tail = red_tail_take<T>();
+    launch_pdl(k_res_flux_pair<T>, fgrid + (tail.n ? 1 : 0), 256, 0, s, E.n,
                reinterpret_cast<const int2 *>(map_dev(ra[0].map)),
-               reinterpret_cast<const int2 *>(map_dev(ra[2].map)), E.xa, E.qa, E.adta, B, vals, K);
+               reinterpret_cast<const int2 *>(map_dev(ra[2].map)), E.xa, E.qa, E.adta, B, vals, K,
+               tail);
+  }
   else if (tuning("flux_pipe", 0))
     launch_pdl(k_res_flux_list<T, true, sizeof(T) == 4 ? 6 : 3>, fgrid, 256, 0, s, E, B, vals, K);
   else
@@ -2532,7 +2655,8 @@ template <class T>
 static bool res_chain_t(char const *loop_name, op_set rset, const op_arg *ra, op_set bset,
                         const op_arg *ba, const op_arg *ua, const op_arg *aa, const op_arg *sa,
                         void *adt_out, void *save_out, bool flux_done,
-                        std::vector<GblRequest> *held, bool res_zero, const ColourKey &key) {
+                        std::vector<GblRequest> *held, bool res_zero, const ColourKey &key,
+                        bool tail_next) {
   // save_soln rides on the one-cell-per-thread fold + update + adt_calc forms
   const int fvar = tuning("fold_variant", 0);
   if (sa && (!ua || !aa || (fvar != 0 && fvar != 4 && fvar != 5))) return false;
@@ -2566,6 +2690,7 @@ static bool res_chain_t(char const *loop_name, op_set rset, const op_arg *ra, op
   // from +0.0 in registers, and res is neither read nor rewritten
   const bool skip_res = res_zero && ua && ua[2].dat == ra[6].dat && tuning("known_zero", 1);
   int rslot_id = ua ? red_new_slot() : -1;
+  unsigned tail_seq = 0;  // the flag of an rms left to the next kernel
   {
     LoopScope ls(name.c_str(), bytes, 0);
     ResEdges<T> E = res_edges<T>(rset, ra);
@@ -2596,11 +2721,11 @@ static bool res_chain_t(char const *loop_name, op_set rset, const op_arg *ra, op
       // 25.6 -> 21.3 us for the fold + update + adt_calc at 720k cells).
       // The grid depends only on ncell and the kernel, so sums reproduce.
       // Knob > 0: that many CTAs per SM; 0: one cell per thread
-      const long long gw = (ncell + 255LL) / 256;
       const int per_sm = aa ? tuning("fold_adt_ctas_per_sm", -1) : tuning("fold_ctas_per_sm", -1);
-      auto grid_of = [&](const void *kernel) {
+      auto grid_of = [&](const void *kernel, int threads = 256) {
+        const long long gw = (ncell + threads - 1LL) / threads;
         long long per = per_sm;
-        if (per < 0) per = resident_ctas(kernel, 256);
+        if (per < 0) per = resident_ctas(kernel, threads);
         long long gcap = per > 0 ? (long long)rt().num_sms * per : (long long)kMaxRedBlocks;
         return (int)std::max(1LL, std::min(gw, std::min(gcap, (long long)kMaxRedBlocks)));
       };
@@ -2641,7 +2766,40 @@ static bool res_chain_t(char const *loop_name, op_set rset, const op_arg *ra, op
 #define OP2B_FOLD_PF(...) launch(k_fold_update_pf<__VA_ARGS__>, k_fold_update_pf<__VA_ARGS__, true>)
 #define OP2B_FOLD_COL(...) \
   launch(k_fold_update<__VA_ARGS__, false, true>, k_fold_update<__VA_ARGS__, true, true>)
-      if (col) {
+      const bool cells =
+          tuning("fold_cells", 1) && W == 4 && fv == 0 &&
+          (!aa || (N.m0.map && N.m0.map == N.m1.map && N.m0.map == N.m2.map &&
+                   N.m0.map == N.m3.map && N.m0.dim == 4 && N.m0.idx == 0 && N.m1.idx == 1 &&
+                   N.m2.idx == 2 && N.m3.idx == 3 && xs[0] == xs[1] && xs[0] == xs[2] &&
+                   xs[0] == xs[3] && (long long)aa[0].dat->set->size < (1LL << 30))) &&
+          (long long)ncell < (1LL << 29) && nval < ((size_t)1 << 29);
+      auto launch_cells = [&](auto kr, auto ks) {
+        auto kernel = skip_res ? ks : kr;
+        const bool leave = !seq && tuning("red_tail", 1) && (rt().gbl_deferred || tail_next);
+        launch_pdl(kernel, grid_of((const void *)kernel, kFoldThreads), kFoldThreads, 0, s, (unsigned)ncell,
+                   reinterpret_cast<const int4 *>(ell), (const T *)vals, qold, q,
+                   skip_res ? (T *)nullptr : res, (const T *)adt,
+                   reinterpret_cast<const int4 *>(N.m0.map), xs[0], K, seqbuf, rslot,
+                   leave ? nullptr : red_ticket(), qsave, adt_to ? adt_to : adt);
+        if (skip_res)
+          zero_entry(ra[6].dat, 5, kernel_nparams(kernel), (const void *)kr,
+                     grid_of((const void *)kr, kFoldThreads));
+        if (leave)
+          tail_seq = red_tail_leave(sizeof(T) == 8 ? GBL_F64 : GBL_F32,
+                                    grid_of((const void *)kernel, kFoldThreads), rslot_id, -1, 12,
+                                    kernel_nparams(kernel));
+      };
+#define OP2B_CELLS(ADT, SAVE, COL) \
+  launch_cells(k_fold_cells<T, ADT, SAVE, false, COL>, k_fold_cells<T, ADT, SAVE, true, COL>)
+      if (cells && col) {
+        if (sa) OP2B_CELLS(true, true, true);
+        else if (aa) OP2B_CELLS(true, false, true);
+        else OP2B_CELLS(false, false, true);
+      } else if (cells) {
+        if (sa) OP2B_CELLS(true, true, false);
+        else if (aa) OP2B_CELLS(true, false, false);
+        else OP2B_CELLS(false, false, false);
+      } else if (col) {
         if (sa) OP2B_FOLD_COL(T, true, 1, sizeof(T) == 4 ? 4 : 2, true);
         else if (aa) OP2B_FOLD_COL(T, true, 1, sizeof(T) == 4 ? 4 : 2, false);
         else OP2B_FOLD_COL(T, false, 1, sizeof(T) == 4 ? 5 : 2, false);
@@ -2665,6 +2823,7 @@ static bool res_chain_t(char const *loop_name, op_set rset, const op_arg *ra, op
         else OP2B_FOLD(T, false, 1, sizeof(T) == 4 ? 5 : 2, false);
       }
 #undef OP2B_FOLD
+#undef OP2B_CELLS
 #undef OP2B_FOLD_PF
 #undef OP2B_FOLD_COL
       if (seq) {
@@ -2678,7 +2837,7 @@ static bool res_chain_t(char const *loop_name, op_set rset, const op_arg *ra, op
   // every update zeroes res, whichever form ran
   if (ua && ua[2].dat == ra[6].dat && !error_pending()) dat_set_known_zero(ra[6].dat, true);
   if (ua) {
-    GblRequest rq{ua[4].data, rslot_id, OP_INC, sizeof(T) == 8 ? GBL_F64 : GBL_F32, seq};
+    GblRequest rq{ua[4].data, rslot_id, OP_INC, sizeof(T) == 8 ? GBL_F64 : GBL_F32, seq, tail_seq};
     if (held) held->push_back(rq);  // the caller delivers it
     else red_finish({rq});
   }
@@ -2700,11 +2859,12 @@ unsigned wait_timeouts(bool reset) {
 bool run_res_chain(char const *name, op_set rset, const op_arg *ra, op_set bset,
                    const op_arg *ba, const op_arg *ua, const op_arg *aa, const op_arg *sa,
                    void *adt_out, void *save_out, bool flux_done,
-                   std::vector<GblRequest> *held, bool res_zero, const ColourKey &key) {
+                   std::vector<GblRequest> *held, bool res_zero, const ColourKey &key,
+                   bool tail_next) {
   return is_double(ra[0]) ? res_chain_t<double>(name, rset, ra, bset, ba, ua, aa, sa, adt_out,
-                                                save_out, flux_done, held, res_zero, key)
+                                                save_out, flux_done, held, res_zero, key, tail_next)
                           : res_chain_t<float>(name, rset, ra, bset, ba, ua, aa, sa, adt_out,
-                                               save_out, flux_done, held, res_zero, key);
+                                               save_out, flux_done, held, res_zero, key, tail_next);
 }
 
 }  // namespace op2b

@@ -169,6 +169,23 @@ __device__ __forceinline__ void add_listed(T r[4], int k, const T f[4]) {
   }
 }
 
+// the same without a branch, for an entry that is there: r + f or r + (-f), as
+// one rounding of (+-1) f + r
+__device__ __forceinline__ float signed_one(int k, float) {
+  return __int_as_float(0x3f800000 | k << 31);
+}
+__device__ __forceinline__ double signed_one(int k, double) {
+  return __hiloint2double(0x3ff00000 | k << 31, 0);
+}
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+template <class T>
+__device__ __forceinline__ void add_signed(T r[4], int k, const T f[4]) {
+  const T s = signed_one(k, T(0));
+#pragma unroll
+  for (int d = 0; d < 4; d++) r[d] = fma_rn(s, f[d], r[d]);
+}
+
 // the same for a list in the order of the two-level colouring (entry = index
 // << 2 | last of its block << 1 | negate; -1: none).  A block's increments of
 // the cell gather in acc from +0, each as 0 + f or 0 - f, and its last adds

@@ -17,7 +17,7 @@
 #include <unordered_set>
 #include <vector>
 
-#include "internal.h"
+#include "loops.h"
 
 void op2b_release_plans();  // plan.cu
 
@@ -541,6 +541,7 @@ void *op2b_get_stream(void) {
 void op2b_set_stream(void *s) {
   ensure_cuda();
   Runtime &R = rt();
+  red_tail_flush();
   if (R.stream && R.stream != (cudaStream_t)s) cudaStreamSynchronize(R.stream);
   R.stream = (cudaStream_t)s;
   R.own_stream = false;

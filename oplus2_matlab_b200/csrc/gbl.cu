@@ -10,9 +10,12 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
+#include <thread>
 
 #include "launch.cuh"
 #include "loops.h"
+#include "reduce.cuh"
 #include "seq_sum.cuh"
 
 namespace op2b {
@@ -24,6 +27,8 @@ struct RedState {
   // result slots in mapped pinned host memory: the last block of a reduction
   // stores the result where the host reads it, so delivery needs no copy
   char *host = nullptr;
+  unsigned *flags = nullptr;  // one per slot, in the same memory
+  unsigned flag_seq = 0;      // the last number given to a flag
   int next_slot = 0;
   int graph_slots = 0;  // slots baked into captured graphs stay reserved
   void *seq = nullptr;
@@ -42,8 +47,9 @@ void ensure_red() {
   size_t bytes = off_slots();
   S.dev = (char *)dev_alloc(bytes);
   OP2B_CUDA(cudaMemset(S.dev, 0, bytes));
-  OP2B_CUDA(cudaHostAlloc((void **)&S.host, (size_t)kSlots * 8, cudaHostAllocMapped));
-  memset(S.host, 0, (size_t)kSlots * 8);
+  OP2B_CUDA(cudaHostAlloc((void **)&S.host, (size_t)kSlots * 12, cudaHostAllocMapped));
+  memset(S.host, 0, (size_t)kSlots * 12);
+  S.flags = (unsigned *)(S.host + (size_t)kSlots * 8);
 }
 
 template <class T>
@@ -60,6 +66,7 @@ void combine(char *host, const T v, op_access acc, bool assign) {
 void deliver(const std::vector<GblRequest> &reqs) {
   RedState &S = rs();
   if (reqs.empty()) return;
+  red_tail_flush();
   int lo = kSlots, hi = -1;
   for (auto &r : reqs) {
     lo = std::min(lo, r.slot);
@@ -79,10 +86,139 @@ std::vector<GblRequest> &pending() {
   static std::vector<GblRequest> v;
   return v;
 }
+
+// with no result outstanding, every slot a captured graph does not hold is free
+void free_slots() {
+  if (pending().empty()) rs().next_slot = rs().graph_slots;
+}
+
+struct Tail {  // red_tail_leave
+  bool on = false, captured = false;
+  int type = 0, n = 0, slot = 0, slot_max = -1, ticket_arg = 0, nparams = 0;
+  unsigned seq = 0;
+  cudaGraphNode_t node = nullptr;
+};
+Tail g_tail;
+std::vector<Tail> g_tail_patches;
+
+template <class T>
+RedTail<T> tail_of(const Tail &t) {
+  RedState &S = rs();
+  RedTail<T> r;
+  r.sums = (const T *)S.dev;
+  r.maxs = t.slot_max >= 0 ? (const T *)(S.dev + (size_t)kMaxRedBlocks * 8) : nullptr;
+  r.sum = (T *)(S.host + (size_t)t.slot * 8);
+  r.max = t.slot_max >= 0 ? (T *)(S.host + (size_t)t.slot_max * 8) : nullptr;
+  r.flag = t.seq ? S.flags + t.slot : nullptr;
+  r.seq = t.seq;
+  r.n = t.n;
+  return r;
+}
+
+template <class T>
+__global__ void __launch_bounds__(256) k_red_tail(RedTail<T> t) {
+  pdl_wait();
+  pdl_trigger();
+  red_tail_fold(t);
+}
+
+// the request's result is in host memory once its flag says so.  A look at
+// the stream from time to time ends the wait when the work behind it failed.
+bool wait_flag(const GblRequest &r) {
+  volatile unsigned *f = rs().flags + r.slot;
+  static const char *yield = getenv("OP2B_SYNC_YIELD");
+  for (unsigned n = 1; *f != r.seq; n++) {
+    if (yield && yield[0] == '1') std::this_thread::yield();
+    if (n & 0x3fff) continue;
+    const cudaError_t e = cudaStreamQuery(rt().stream);
+    if (e == cudaErrorNotReady) continue;
+    if (e == cudaSuccess && *f == r.seq) break;
+    cuda_fail(e == cudaSuccess ? cudaErrorUnknown : e, "global reduction", __FILE__, __LINE__);
+    return false;
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  return true;
+}
 }  // namespace
 
+unsigned red_tail_leave(int type, int n, int slot, int slot_max, int ticket_arg, int nparams) {
+  Tail t;
+  t.on = true;
+  t.type = type;
+  t.n = n;
+  t.slot = slot;
+  t.slot_max = slot_max;
+  t.ticket_arg = ticket_arg;
+  t.nparams = nparams;
+  if (!rt().gbl_deferred) {
+    if (++rs().flag_seq == 0) ++rs().flag_seq;
+    t.seq = rs().flag_seq;
+  }
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  const cudaGraphNode_t *deps = nullptr;
+  const cudaGraphEdgeData *edges = nullptr;
+  size_t nd = 0;
+  if (rt().gbl_deferred &&
+      cudaStreamGetCaptureInfo_v3(rt().stream, &st, nullptr, nullptr, &deps, &edges, &nd) ==
+          cudaSuccess &&
+      st == cudaStreamCaptureStatusActive) {
+    t.captured = true;
+    cudaGraphNodeType kind;
+    if (nd == 1 && cudaGraphNodeGetType(deps[0], &kind) == cudaSuccess &&
+        kind == cudaGraphNodeTypeKernel)
+      t.node = deps[0];
+  }
+  cudaGetLastError();
+  g_tail = t;
+  return t.seq;
+}
+
+template <class T>
+RedTail<T> red_tail_take() {
+  if (g_tail.on && g_tail.type == (sizeof(T) == 8 ? GBL_F64 : GBL_F32)) {
+    g_tail.on = false;
+    return tail_of<T>(g_tail);
+  }
+  RedTail<T> none;
+  memset(&none, 0, sizeof none);
+  return none;
+}
+template RedTail<float> red_tail_take<float>();
+template RedTail<double> red_tail_take<double>();
+
+void red_tail_flush() {
+  if (!g_tail.on) return;
+  g_tail.on = false;
+  if (g_tail.captured && g_tail.node) {  // that kernel folds its partials itself
+    g_tail_patches.push_back(g_tail);
+    return;
+  }
+  if (g_tail.type == GBL_F64)
+    launch_pdl(k_red_tail<double>, 1, 256, 0, rt().stream, tail_of<double>(g_tail));
+  else
+    launch_pdl(k_red_tail<float>, 1, 256, 0, rt().stream, tail_of<float>(g_tail));
+}
+
+void red_tail_patch_captured() {
+  for (Tail &t : g_tail_patches) {
+    cudaKernelNodeParams kp;
+    OP2B_CUDA(cudaGraphKernelNodeGetParams(t.node, &kp));
+    if (error_pending()) break;
+    std::vector<void *> args(kp.kernelParams, kp.kernelParams + t.nparams);
+    unsigned *ticket = red_ticket();
+    args[t.ticket_arg] = &ticket;
+    kp.kernelParams = args.data();
+    kp.extra = nullptr;
+    OP2B_CUDA(cudaGraphKernelNodeSetParams(t.node, &kp));
+  }
+  g_tail_patches.clear();
+}
+
+// every reduction asks for its partials before it is launched: those of the
+// one before it are folded by then
 void *red_partials(int i) {
   ensure_red();
+  red_tail_flush();
   return rs().dev + (size_t)i * kMaxRedBlocks * 8;
 }
 
@@ -158,19 +294,22 @@ void red_finish(const std::vector<GblRequest> &reqs) {
     return;
   }
   deliver(reqs);
-  if (pending().empty() && rs().graph_slots == 0) rs().next_slot = 0;
+  free_slots();
 }
 
 void red_finish_after(cudaEvent_t done, const std::vector<GblRequest> &reqs) {
   if (reqs.empty()) return;
   RedState &S = rs();
-  OP2B_CUDA(cudaEventSynchronize(done));  // the slots are host memory
+  bool event = false;
+  for (auto &r : reqs) event = event || !r.seq;
+  if (event) OP2B_CUDA(cudaEventSynchronize(done));  // the slots are host memory
   for (auto &r : reqs) {
+    if (r.seq && !wait_flag(r)) return;
     const char *p = S.host + (size_t)r.slot * 8;
     if (r.type == GBL_F64) combine<double>(r.host, *(const double *)p, r.acc, r.assign);
     else combine<float>(r.host, *(const float *)p, r.acc, r.assign);
   }
-  if (pending().empty() && S.graph_slots == 0) S.next_slot = 0;
+  free_slots();
 }
 
 size_t red_pending_count() { return pending().size(); }
@@ -202,7 +341,7 @@ void deliver_deferred() {
   std::vector<GblRequest> v;
   v.swap(pending());
   deliver(v);
-  if (rs().graph_slots == 0) rs().next_slot = 0;
+  free_slots();
 }
 
 void red_reserve_for_graph() { rs().graph_slots = std::max(rs().graph_slots, rs().next_slot); }

@@ -122,6 +122,7 @@ int op2b_capture_begin(int profile) {
   if (error_pending()) return 0;
   Runtime &R = rt();
   flush_pending();  // loops held back before the capture run outside the graph
+  red_tail_flush();
   ahead_drop();     // a graph bakes dataset pointers: nothing may be swapped in later
   tile_capture_begin();
   known_zero_capture_begin();
@@ -145,6 +146,7 @@ int op2b_capture_begin(int profile) {
 
 void *op2b_capture_end(void) {
   flush_pending();
+  red_tail_flush();
   tile_capture_end();  // the graph leaves every dataset in the buffer it found
   Runtime &R = rt();
   Graph *g = new Graph();
@@ -160,6 +162,7 @@ void *op2b_capture_end(void) {
     fail(-1, "op2b error: graph capture failed: %s\n", cudaGetErrorString(e));
     return nullptr;
   }
+  red_tail_patch_captured();
   g->loops.swap(R.capture_events);
   size_t n = 0;
   OP2B_CUDA(cudaGraphGetNodes(g->graph, nullptr, &n));
@@ -185,6 +188,7 @@ int op2b_graph_launch(void *h) {
   Graph *g = (Graph *)h;
   if (!g) return (int)cudaErrorInvalidValue;
   if (!zero_entries_match(g)) return -1;
+  red_tail_flush();  // the graph's reductions write the same partials
   red_replace_pending(g->reductions);
   const cudaError_t e = cudaGraphLaunch(g->exec, rt().stream);
   if (e == cudaSuccess) known_zero_apply(g->zero_effects);

@@ -342,29 +342,32 @@ bool run_chain_ahead(const std::vector<Held> &ch) {
   void *adt_out = spare_of(g_seen_adt[5].dat);
   void *save_out = save ? spare_of(g_seen_save[1].dat) : nullptr;
   if (error_pending()) return false;
-  std::vector<GblRequest> held;
-  if (!run_res_chain(nullptr, ch[0].set, ch[0].args.data(), ch[1].set, ch[1].args.data(), ua,
-                     g_seen_adt.data(), save ? g_seen_save.data() : nullptr, adt_out, save_out,
-                     ch[0].flux_done, &held, ch[0].res_zero, colour_key(ch)))
-    return false;
-  g_ahead.adt = true;
-  g_ahead.save = save;
-  g_ahead.adt_args = g_seen_adt;
-  g_ahead.save_args = g_seen_save;
-  g_ahead.consts_version = rt().consts_version;
-  // the next chain's flux pass, behind an event that marks this update done
+  // the next chain's flux pass is queued behind this update's (below)
   const bool next = tuning("flux_ahead", 1) && g_seen_res.size() == 8 &&
                     g_seen_bres.size() == 6 && g_seen_res[2].dat == ua[1].dat &&
                     g_seen_res[3].dat == ua[1].dat && g_seen_res[4].dat == ua[3].dat &&
                     g_seen_res[5].dat == ua[3].dat && g_seen_res[6].dat == ua[2].dat &&
                     bres_follows_res(g_seen_res.data(), g_seen_bres.data()) &&
                     g_seen_adt[5].dat == ua[3].dat;
+  std::vector<GblRequest> held;
+  if (!run_res_chain(nullptr, ch[0].set, ch[0].args.data(), ch[1].set, ch[1].args.data(), ua,
+                     g_seen_adt.data(), save ? g_seen_save.data() : nullptr, adt_out, save_out,
+                     ch[0].flux_done, &held, ch[0].res_zero, colour_key(ch), next))
+    return false;
+  g_ahead.adt = true;
+  g_ahead.save = save;
+  g_ahead.adt_args = g_seen_adt;
+  g_ahead.save_args = g_seen_save;
+  g_ahead.consts_version = rt().consts_version;
+  // the next chain's flux pass, which also folds the rms left to it, or
+  // behind an event that marks this update done
   if (!next) {
     red_finish(held);
     return true;
   }
+  const bool flagged = held.size() == 1 && held[0].seq;
   if (!g_fold_done) OP2B_CUDA(cudaEventCreateWithFlags(&g_fold_done, cudaEventDisableTiming));
-  OP2B_CUDA(cudaEventRecord(g_fold_done, rt().stream));
+  if (!flagged) OP2B_CUDA(cudaEventRecord(g_fold_done, rt().stream));
   g_next = NextFlux();
   g_next.valid = run_res_flux_ahead(g_seen_res_set, g_seen_res.data(), g_seen_bres_set,
                                     g_seen_bres.data(), ua[3].dat, adt_out);
@@ -373,6 +376,7 @@ bool run_chain_ahead(const std::vector<Held> &ch) {
   g_next.res_set = g_seen_res_set;
   g_next.bres_set = g_seen_bres_set;
   g_next.consts_version = rt().consts_version;
+  red_tail_flush();  // when no flux pass took the rms
   red_finish_after(g_fold_done, held);
   return true;
 }

@@ -40,6 +40,7 @@ struct GblRequest {
   op_access acc;
   int type;        // GblType
   bool assign;     // SEQ-mode sum: device value already includes the seed
+  unsigned seq = 0;  // not 0: the slot's flag has this value once the result is there
 };
 constexpr int kMaxRedBlocks = 4096;
 void *red_partials(int i);       // [kMaxRedBlocks] of 8-byte entries, i in {0,1}
@@ -51,8 +52,24 @@ void *red_seq_buffer(size_t bytes);  // scratch for SEQ-mode contributions
 // renumbered set: see SeqVals); v is red_seq_buffer's
 template <class T>
 void seq_sum(const T *v, long long n, T init, T *out, const int *order, int w);
+// The kernel just launched wrote its n block partials (in red_partials) of a
+// sum, and of a maximum when slot_max >= 0, and left them unfolded: the next
+// kernel that takes the tail folds them, or red_tail_flush does.  Returns the
+// number the slot's flag will have (0 with deferred reductions).  ticket_arg:
+// the kernel's parameter that makes it fold its partials itself, given a
+// ticket (of nparams parameters), for a capture that ends before another
+// kernel takes the tail.
+unsigned red_tail_leave(int type, int n, int slot, int slot_max, int ticket_arg, int nparams);
+template <class T>
+struct RedTail;
+template <class T>
+RedTail<T> red_tail_take();  // n == 0: none, or of the other type
+void red_tail_flush();
+// at the end of a capture: the kernels that now fold their own partials
+void red_tail_patch_captured();
 void red_finish(const std::vector<GblRequest> &reqs);
-// the same, waiting only for the work up to the event (not deferred mode)
+// the same, waiting only for the work up to the event, or for the requests'
+// flags when they have them (not deferred mode)
 void red_finish_after(cudaEvent_t done, const std::vector<GblRequest> &reqs);
 // deferred requests (graph capture): count, take those added since a mark,
 // and re-arm a set (replacing any pending request on the same slots)
@@ -118,6 +135,7 @@ bool run_res_bres(op_set res_set, const op_arg *res_args, op_set bres_set,
 // flux_done: the flux pass already ran for exactly these arguments (run
 // ahead, run_res_flux_ahead).  held: the update's reduction is appended
 // there for the caller to deliver, instead of being delivered here.
+// tail_next: a flux pass follows at once, so the rms may be left to it.
 // res_zero: res held +0.0 in every element when res_calc was called (then,
 // with update, res is neither read nor rewritten).
 bool run_res_chain(char const *name, op_set res_set, const op_arg *res_args, op_set bres_set,
@@ -125,7 +143,7 @@ bool run_res_chain(char const *name, op_set res_set, const op_arg *res_args, op_
                    const op_arg *save_args = nullptr, void *adt_out = nullptr,
                    void *save_out = nullptr, bool flux_done = false,
                    std::vector<GblRequest> *held = nullptr, bool res_zero = false,
-                   const ColourKey &key = ColourKey());
+                   const ColourKey &key = ColourKey(), bool tail_next = false);
 // the flux pass of a res_calc + bres_calc chain before its calls, adt read
 // from adt_now instead of adt's buffer; false when not applicable
 bool run_res_flux_ahead(op_set res_set, const op_arg *res_args, op_set bres_set,

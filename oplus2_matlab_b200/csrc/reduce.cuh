@@ -16,6 +16,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <math.h>
 
 namespace op2b {
 
@@ -93,6 +94,53 @@ __device__ __forceinline__ void grid_finish(const T (&v)[N], const T (&identity)
     if (threadIdx.x == 0) *slot[i].result = x;
   }
   if (threadIdx.x == 0) *ticket = 0u;
+}
+
+// The end of a reduction left to another kernel: the block partials of one
+// or two reductions (a sum, and a maximum) that a kernel has written and not
+// folded.  Folding them in that kernel's last block keeps the next kernel
+// waiting for a chain of fence, ticket, loads and a store to host memory
+// (2 us at the end of every res_calc chain); a CTA of the next kernel does it
+// while the others work.  flag, when not null, is set to seq once the results
+// are in host memory, for a host that waits for them.
+template <class T>
+struct RedTail {
+  const T *sums, *maxs;  // [n]; maxs may be null
+  T *sum, *max;
+  unsigned *flag, seq;
+  int n;  // 0: nothing to do
+};
+
+// by all threads of a block
+template <class T>
+__device__ __forceinline__ void red_tail_fold(const RedTail<T> &t) {
+  __shared__ T ws[32];
+  const T low = -static_cast<T>(INFINITY);
+  T x = T(0), y = low;
+  for (int k0 = threadIdx.x; k0 < t.n; k0 += 4 * blockDim.x) {
+    T a[4], b[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {  // the loads of a round together
+      const int k = k0 + i * blockDim.x;
+      a[i] = k < t.n ? __ldcg(t.sums + k) : T(0);
+      b[i] = t.maxs && k < t.n ? __ldcg(t.maxs + k) : low;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      x += a[i];
+      y = OpMax()(y, b[i]);
+    }
+  }
+  x = block_fold(x, T(0), OpSum(), ws);
+  if (t.maxs) y = block_fold(y, low, OpMax(), ws);
+  if (threadIdx.x == 0) {
+    *t.sum = x;
+    if (t.maxs) *t.max = y;
+    if (t.flag) {
+      __threadfence_system();
+      *reinterpret_cast<volatile unsigned *>(t.flag) = t.seq;
+    }
+  }
 }
 
 }  // namespace op2b
