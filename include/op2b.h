@@ -62,6 +62,11 @@ enum { OP2B_REDUCE_TREE = 0, OP2B_REDUCE_SEQ = 1 };
  *                   the res that follows it as one launch ("jac_tile_nodes"
  *                   the tile size, 0 automatic; "jac_step_threads" 512,
  *                   1024 or 256 per CTA); 0: two launches
+ *   "fold_cells"    1 (default): the per-cell pass of the airfoil shape (lists
+ *                   of four, one x dataset) with every load of a thread's next
+ *                   cell ahead of this cell's arithmetic; 0: the general pass
+ *   "red_tail"      1 (default): the rms of an update is folded by the flux
+ *                   pass behind it; 0: by the update's last block
  *   "coloured_fold" 1 (default): COLOURED res_calc [+ bres_calc ...] as the
  *                   flux pass and a per-cell fold in the plan's order; 0: one
  *                   launch per block colour

@@ -650,6 +650,12 @@ __global__ void __launch_bounds__(256, MINB)
 // load of a thread's next cell -- its own streams, its nodes and its listed
 // values -- is issued before this cell's arithmetic, and the indices two cells
 // ahead, so a warp has a cell's loads in flight while it computes.
+// Bound: the latency of the gathers (ten of the eighteen cycles a warp spends
+// per instruction in the general form).  Registers pay for the loads in
+// flight, not for warps: 2 CTAs of 256 per SM (FP64 1) beat 3 and 4, which
+// spill (iteration 47.1 against 55.4 and 63.6 us at 720k FP32), and 128-thread
+// CTAs, whose partials take longer to fold (48.0).  Against the general form:
+// 49.1 -> 47.1 us an iteration at 720k FP32, 57.3 -> 54.1 at 407k FP64.
 template <class T>
 struct CellIn {
   T f[4][4], x[4][2], qo[4], r[4], ad;
@@ -743,7 +749,7 @@ __global__ void __launch_bounds__(kFoldThreads, sizeof(T) == 4 ? 2 : 1)
     c += stride;
   }
   if (seq) return;
-  if (!ticket) {  // the next kernel folds the partials
+  if (!ticket) {  // the next kernel folds the partials (RedTail)
     __shared__ T ws[32];
     rms = block_fold(rms, T(0), OpSum(), ws);
     if (threadIdx.x == 0) slot.partials[blockIdx.x] = rms;

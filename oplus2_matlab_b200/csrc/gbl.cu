@@ -122,7 +122,9 @@ __global__ void __launch_bounds__(256) k_red_tail(RedTail<T> t) {
   red_tail_fold(t);
 }
 
-// the request's result is in host memory once its flag says so.  A look at
+// The request's result is in host memory once its flag says so, which is
+// before an event behind the kernel would be seen (eager iteration at 7k cells
+// 41.5 -> 35.1 us, at 720k 62.9 -> 54.4, relieved kernels included).  A look at
 // the stream from time to time ends the wait when the work behind it failed.
 bool wait_flag(const GblRequest &r) {
   volatile unsigned *f = rs().flags + r.slot;
