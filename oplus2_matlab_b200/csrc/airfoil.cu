@@ -749,15 +749,10 @@ __global__ void __launch_bounds__(kFoldThreads, sizeof(T) == 4 ? 2 : 1)
     c += stride;
   }
   if (seq) return;
-  if (!ticket) {  // the next kernel folds the partials (RedTail)
-    __shared__ T ws[32];
-    rms = block_fold(rms, T(0), OpSum(), ws);
-    if (threadIdx.x == 0) slot.partials[blockIdx.x] = rms;
-    return;
-  }
   const T v[1] = {rms}, id[1] = {T(0)};
   RedSlot<T> sl[1] = {slot};
-  grid_finish<T, OpSum, OpSum, 1>(v, id, OpSum(), OpSum(), sl, ticket);
+  if (!ticket) grid_leave<T, OpSum, OpSum, 1>(v, id, OpSum(), OpSum(), sl);
+  else grid_finish<T, OpSum, OpSum, 1>(v, id, OpSum(), OpSum(), sl, ticket);
 }
 
 // One cell per thread, with the cell's own streams (res, qold, adt) fetched
@@ -1535,6 +1530,7 @@ static void update_t(char const *name, op_set set, const op_arg *args) {
   const bool seq = rt().reduction == OP2B_REDUCE_SEQ;
   int slot = red_new_slot();
   T *result = (T *)red_slot_ptr(slot);
+  unsigned flag_seq = 0;
   {
     LoopScope ls(name, compulsory_bytes(set, 5, args), 0);
     T *seqbuf = seq ? (T *)red_seq_buffer(sizeof(T) * 4 * (size_t)n) : nullptr;
@@ -1546,6 +1542,7 @@ static void update_t(char const *name, op_set set, const op_arg *args) {
     long long gcap = (long long)rt().num_sms * tuning("update_ctas_per_sm", 4);
     const int grid = (int)std::max(1LL, std::min(gw, std::min(gcap, (long long)kMaxRedBlocks)));
     RedSlot<T> rslot{(T *)red_partials(0), result};
+    if (!seq) rslot.seq = flag_seq = red_flag(slot, &rslot.flag);
     const T *qold = (const T *)args[0].dat->data_d, *adt = (const T *)args[3].dat->data_d;
     T *q = (T *)args[1].dat->data_d, *res = (T *)args[2].dat->data_d;
     auto launch = [&](auto kernel) {
@@ -1559,7 +1556,8 @@ static void update_t(char const *name, op_set set, const op_arg *args) {
       seq_sum<T>(seqbuf, 4LL * n, init, result, perm_old2new_dev(set), 4);
     }
   }
-  red_finish({GblRequest{args[4].data, slot, OP_INC, sizeof(T) == 8 ? GBL_F64 : GBL_F32, seq}});
+  red_finish({GblRequest{args[4].data, slot, OP_INC, sizeof(T) == 8 ? GBL_F64 : GBL_F32, seq,
+                         flag_seq, slot}});
 }
 void run_airfoil_update(char const *name, op_set set, const op_arg *args) {
   if (is_double(args[0])) update_t<double>(name, set, args);
@@ -2759,6 +2757,7 @@ static bool res_chain_t(char const *loop_name, op_set rset, const op_arg *ra, op
       auto launch = [&](auto kr, auto ks) {
         const bool skip = skip_res;
         auto kernel = skip ? ks : kr;
+        if (!seq) rslot.seq = tail_seq = red_flag(rslot_id, &rslot.flag);
         launch_pdl(kernel, grid_of((const void *)kernel), 256, 0, s, ncell,
                    ell, W, (const T *)vals,
                    qold, q, skip ? (T *)nullptr : res, adt, N, xs[0], xs[1], xs[2], xs[3],
@@ -2782,6 +2781,7 @@ static bool res_chain_t(char const *loop_name, op_set rset, const op_arg *ra, op
       auto launch_cells = [&](auto kr, auto ks) {
         auto kernel = skip_res ? ks : kr;
         const bool leave = !seq && tuning("red_tail", 1) && (rt().gbl_deferred || tail_next);
+        if (!leave && !seq) rslot.seq = tail_seq = red_flag(rslot_id, &rslot.flag);
         launch_pdl(kernel, grid_of((const void *)kernel, kFoldThreads), kFoldThreads, 0, s, (unsigned)ncell,
                    reinterpret_cast<const int4 *>(ell), (const T *)vals, qold, q,
                    skip_res ? (T *)nullptr : res, (const T *)adt,
@@ -2843,7 +2843,7 @@ static bool res_chain_t(char const *loop_name, op_set rset, const op_arg *ra, op
   // every update zeroes res, whichever form ran
   if (ua && ua[2].dat == ra[6].dat && !error_pending()) dat_set_known_zero(ra[6].dat, true);
   if (ua) {
-    GblRequest rq{ua[4].data, rslot_id, OP_INC, sizeof(T) == 8 ? GBL_F64 : GBL_F32, seq, tail_seq};
+    GblRequest rq{ua[4].data, rslot_id, OP_INC, sizeof(T) == 8 ? GBL_F64 : GBL_F32, seq, tail_seq, rslot_id};
     if (held) held->push_back(rq);  // the caller delivers it
     else red_finish({rq});
   }

@@ -63,19 +63,35 @@ void combine(char *host, const T v, op_access acc, bool assign) {
   }
 }
 
+// The request's result is in host memory once its flag says so, which is
+// before an event behind the kernel would be seen (eager iteration at 7k cells
+// 41.5 -> 35.1 us, at 720k 62.9 -> 54.4, relieved kernels included).  A look at
+// the stream from time to time ends the wait when the work behind it failed.
+bool wait_flag(const GblRequest &r) {
+  volatile unsigned *f = rs().flags + r.flag_slot;
+  static const char *yield = getenv("OP2B_SYNC_YIELD");
+  for (unsigned n = 1; *f != r.seq; n++) {
+    if (yield && yield[0] == '1') std::this_thread::yield();
+    if (n & 0x3fff) continue;
+    const cudaError_t e = cudaStreamQuery(rt().stream);
+    if (e == cudaErrorNotReady) continue;
+    if (e == cudaSuccess && *f == r.seq) break;
+    cuda_fail(e == cudaSuccess ? cudaErrorUnknown : e, "global reduction", __FILE__, __LINE__);
+    return false;
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  return true;
+}
+
 void deliver(const std::vector<GblRequest> &reqs) {
   RedState &S = rs();
   if (reqs.empty()) return;
   red_tail_flush();
-  int lo = kSlots, hi = -1;
+  bool sync = false;
+  for (auto &r : reqs) sync = sync || !r.seq;
+  if (sync) OP2B_CUDA(cudaStreamSynchronize(rt().stream));  // the slots are host memory
   for (auto &r : reqs) {
-    lo = std::min(lo, r.slot);
-    hi = std::max(hi, r.slot);
-  }
-  (void)lo;
-  (void)hi;
-  OP2B_CUDA(cudaStreamSynchronize(rt().stream));  // the slots are host memory
-  for (auto &r : reqs) {
+    if (r.seq && !wait_flag(r)) return;
     const char *p = S.host + (size_t)r.slot * 8;
     if (r.type == GBL_F64) combine<double>(r.host, *(const double *)p, r.acc, r.assign);
     else combine<float>(r.host, *(const float *)p, r.acc, r.assign);
@@ -122,26 +138,16 @@ __global__ void __launch_bounds__(256) k_red_tail(RedTail<T> t) {
   red_tail_fold(t);
 }
 
-// The request's result is in host memory once its flag says so, which is
-// before an event behind the kernel would be seen (eager iteration at 7k cells
-// 41.5 -> 35.1 us, at 720k 62.9 -> 54.4, relieved kernels included).  A look at
-// the stream from time to time ends the wait when the work behind it failed.
-bool wait_flag(const GblRequest &r) {
-  volatile unsigned *f = rs().flags + r.slot;
-  static const char *yield = getenv("OP2B_SYNC_YIELD");
-  for (unsigned n = 1; *f != r.seq; n++) {
-    if (yield && yield[0] == '1') std::this_thread::yield();
-    if (n & 0x3fff) continue;
-    const cudaError_t e = cudaStreamQuery(rt().stream);
-    if (e == cudaErrorNotReady) continue;
-    if (e == cudaSuccess && *f == r.seq) break;
-    cuda_fail(e == cudaSuccess ? cudaErrorUnknown : e, "global reduction", __FILE__, __LINE__);
-    return false;
-  }
-  std::atomic_thread_fence(std::memory_order_acquire);
-  return true;
-}
 }  // namespace
+
+unsigned red_flag(int slot, unsigned **flag) {
+  *flag = nullptr;
+  if (rt().gbl_deferred) return 0;
+  RedState &S = rs();
+  if (++S.flag_seq == 0) ++S.flag_seq;
+  *flag = S.flags + slot;
+  return S.flag_seq;
+}
 
 unsigned red_tail_leave(int type, int n, int slot, int slot_max, int ticket_arg, int nparams) {
   Tail t;
@@ -152,10 +158,8 @@ unsigned red_tail_leave(int type, int n, int slot, int slot_max, int ticket_arg,
   t.slot_max = slot_max;
   t.ticket_arg = ticket_arg;
   t.nparams = nparams;
-  if (!rt().gbl_deferred) {
-    if (++rs().flag_seq == 0) ++rs().flag_seq;
-    t.seq = rs().flag_seq;
-  }
+  unsigned *flag;
+  t.seq = red_flag(slot, &flag);
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   const cudaGraphNode_t *deps = nullptr;
   const cudaGraphEdgeData *edges = nullptr;

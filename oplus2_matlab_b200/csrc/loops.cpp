@@ -392,19 +392,23 @@ bool jac_update_ahead(char const *name, op_set set, const op_arg *a, int variant
   void *du_out = spare_of(a[1].dat);
   if (error_pending()) return false;
   std::vector<GblRequest> held;
-  run_jac_update(name, set, a, variant, &held);
+  run_jac_update(name, set, a, variant, &held, true);
   if (error_pending()) {
+    red_tail_flush();
     red_finish(held);
     return true;
   }
+  bool flagged = true;
+  for (auto &r : held) flagged = flagged && r.seq;
   if (!g_fold_done) OP2B_CUDA(cudaEventCreateWithFlags(&g_fold_done, cudaEventDisableTiming));
-  OP2B_CUDA(cudaEventRecord(g_fold_done, rt().stream));
+  if (!flagged) OP2B_CUDA(cudaEventRecord(g_fold_done, rt().stream));
   g_jnext = JacNext();
   g_jnext.beta = *(const float *)g_seen_jres[3].data;  // the value the run uses
   g_jnext.valid = run_jac_res_ahead(g_seen_jres_name.c_str(), g_seen_jres_set,
                                     g_seen_jres.data(), 1, du_out);
   g_jnext.args = g_seen_jres;
   g_jnext.set = g_seen_jres_set;
+  red_tail_flush();  // when no res took the sums
   red_finish_after(g_fold_done, held);
   return true;
 }

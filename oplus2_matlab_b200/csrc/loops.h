@@ -40,13 +40,17 @@ struct GblRequest {
   op_access acc;
   int type;        // GblType
   bool assign;     // SEQ-mode sum: device value already includes the seed
-  unsigned seq = 0;  // not 0: the slot's flag has this value once the result is there
+  unsigned seq = 0;  // not 0: flag_slot's flag has this value once the result is there
+  int flag_slot = 0;
 };
 constexpr int kMaxRedBlocks = 4096;
 void *red_partials(int i);       // [kMaxRedBlocks] of 8-byte entries, i in {0,1}
 unsigned *red_ticket();
 void *red_slot_ptr(int slot);    // 8-byte device slot
 int red_new_slot();
+// a slot's flag and the number a kernel is to set it to when its results are
+// there; null and 0 with deferred reductions
+unsigned red_flag(int slot, unsigned **flag);
 void *red_seq_buffer(size_t bytes);  // scratch for SEQ-mode contributions
 // *out = init + v[0] + v[1] + ... + v[n-1], added in that order (value j of a
 // renumbered set: see SeqVals); v is red_seq_buffer's
@@ -87,9 +91,10 @@ void run_res_calc(char const *name, op_set set, const op_arg *args);
 void run_bres_calc(char const *name, op_set set, const op_arg *args);
 void run_airfoil_update(char const *name, op_set set, const op_arg *args);
 void run_jac_res(char const *name, op_set set, const op_arg *args, int variant);
-// held: the reductions are appended there for the caller to deliver
+// held: the reductions are appended there for the caller to deliver;
+// tail_next: a res follows at once, so they may be left to it
 void run_jac_update(char const *name, op_set set, const op_arg *args, int variant,
-                    std::vector<GblRequest> *held = nullptr);
+                    std::vector<GblRequest> *held = nullptr, bool tail_next = false);
 // jac1's res into du_out (a spare buffer of du's size) instead of du, ahead
 // of its call; false when not applicable (nothing launched)
 // jac1's update followed by its res as one launch (jac.cu); false when the

@@ -60,6 +60,9 @@ template <class T>
 struct RedSlot {
   T *partials;         // [gridDim.x]
   T *result;           // final value (no host seed applied)
+  // the first reduction's: set to seq once every result is in host memory,
+  // for a host that waits for it (null: nobody does)
+  unsigned *flag = nullptr, seq = 0;
 };
 
 // Finish up to two reductions of one kernel: write block partials, and let
@@ -93,7 +96,25 @@ __device__ __forceinline__ void grid_finish(const T (&v)[N], const T (&identity)
     x = i == 0 ? block_fold(x, identity[i], op0, ws) : block_fold(x, identity[i], op1, ws);
     if (threadIdx.x == 0) *slot[i].result = x;
   }
-  if (threadIdx.x == 0) *ticket = 0u;
+  if (threadIdx.x == 0) {
+    *ticket = 0u;
+    if (slot[0].flag) {
+      __threadfence_system();
+      *reinterpret_cast<volatile unsigned *>(slot[0].flag) = slot[0].seq;
+    }
+  }
+}
+
+// a kernel whose partials the next kernel folds (RedTail) writes them only
+template <class T, class Op0, class Op1, int N>
+__device__ __forceinline__ void grid_leave(const T (&v)[N], const T (&identity)[N], Op0 op0,
+                                           Op1 op1, RedSlot<T> (&slot)[N]) {
+  __shared__ T ws[32];
+#pragma unroll
+  for (int i = 0; i < N; i++) {
+    T b = i == 0 ? block_fold(v[i], identity[i], op0, ws) : block_fold(v[i], identity[i], op1, ws);
+    if (threadIdx.x == 0) slot[i].partials[blockIdx.x] = b;
+  }
 }
 
 // The end of a reduction left to another kernel: the block partials of one
