@@ -2780,7 +2780,7 @@ static bool res_chain_t(char const *loop_name, op_set rset, const op_arg *ra, op
           (long long)ncell < (1LL << 29) && nval < ((size_t)1 << 29);
       auto launch_cells = [&](auto kr, auto ks) {
         auto kernel = skip_res ? ks : kr;
-        const bool leave = !seq && tuning("red_tail", 1) && (rt().gbl_deferred || tail_next);
+        const bool leave = !seq && red_tail_wanted(tail_next);
         if (!leave && !seq) rslot.seq = tail_seq = red_flag(rslot_id, &rslot.flag);
         launch_pdl(kernel, grid_of((const void *)kernel, kFoldThreads), kFoldThreads, 0, s, (unsigned)ncell,
                    reinterpret_cast<const int4 *>(ell), (const T *)vals, qold, q,

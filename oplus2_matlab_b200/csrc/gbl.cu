@@ -149,6 +149,15 @@ unsigned red_flag(int slot, unsigned **flag) {
   return S.flag_seq;
 }
 
+bool red_tail_wanted(bool tail_next) {
+  if (!tuning("red_tail", 1)) return false;
+  if (!rt().gbl_deferred) return tail_next;
+  if (rt().own_capture) return true;
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  OP2B_CUDA(cudaStreamIsCapturing(rt().stream, &st));
+  return st == cudaStreamCaptureStatusNone;
+}
+
 unsigned red_tail_leave(int type, int n, int slot, int slot_max, int ticket_arg, int nparams) {
   Tail t;
   t.on = true;
@@ -164,7 +173,7 @@ unsigned red_tail_leave(int type, int n, int slot, int slot_max, int ticket_arg,
   const cudaGraphNode_t *deps = nullptr;
   const cudaGraphEdgeData *edges = nullptr;
   size_t nd = 0;
-  if (rt().gbl_deferred &&
+  if (rt().own_capture &&
       cudaStreamGetCaptureInfo_v3(rt().stream, &st, nullptr, nullptr, &deps, &edges, &nd) ==
           cudaSuccess &&
       st == cudaStreamCaptureStatusActive) {

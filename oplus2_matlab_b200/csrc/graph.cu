@@ -133,9 +133,11 @@ int op2b_capture_begin(int profile) {
   R.capture_profile = profile != 0;
   g_prev_deferred = R.gbl_deferred;
   R.gbl_deferred = true;
+  R.own_capture = true;
   cudaError_t e = cudaStreamBeginCapture(R.stream, cudaStreamCaptureModeRelaxed);
   if (e != cudaSuccess) {
     R.gbl_deferred = g_prev_deferred;
+    R.own_capture = false;
     R.capture_profile = false;
     known_zero_capture_end();
     fail(-1, "op2b error: cannot start graph capture: %s\n", cudaGetErrorString(e));
@@ -154,6 +156,7 @@ void *op2b_capture_end(void) {
   g->zero_entries.swap(g_capture_zero_entries);
   cudaError_t e = cudaStreamEndCapture(R.stream, &g->graph);
   R.capture_profile = false;
+  R.own_capture = false;
   R.gbl_deferred = g_prev_deferred;
   g->reductions = red_take_pending_since(g_pending_mark);
   red_reserve_for_graph();

@@ -92,6 +92,7 @@ struct Runtime {
   // stream capture in progress (graph.cu): per-loop event pairs recorded
   // into the graph when profiling
   bool capture_profile = false;
+  bool own_capture = false;  // between op2b_capture_begin and op2b_capture_end
   struct CapturedLoop {
     std::string name;
     cudaEvent_t start, stop;

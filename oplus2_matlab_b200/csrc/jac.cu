@@ -335,7 +335,7 @@ static void jac_update_t(char const *name, op_set set, const op_arg *args,
     const int threads = 256, grid = red_grid(n, threads);
     // the sum and the maximum are left to the res that follows, at once or,
     // with deferred reductions, in all likelihood
-    const bool leave = !seq && tuning("red_tail", 1) && (rt().gbl_deferred || tail_next);
+    const bool leave = !seq && red_tail_wanted(tail_next);
     RedSlot<float> ss{(float *)red_partials(0), r_sum}, sm{(float *)red_partials(1), r_max};
     if (!leave && !seq) ss.seq = flag_seq = red_flag(slot_sum, &ss.flag);
     launch_pdl(k_jac_update<V>, grid, threads, 0, s, n, (const float *)args[0].dat->data_d,

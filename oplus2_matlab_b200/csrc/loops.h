@@ -63,6 +63,8 @@ void seq_sum(const T *v, long long n, T init, T *out, const int *order, int w);
 // the kernel's parameter that makes it fold its partials itself, given a
 // ticket (of nparams parameters), for a capture that ends before another
 // kernel takes the tail.
+// Not in a caller's own stream capture, which ends without the library.
+bool red_tail_wanted(bool tail_next);
 unsigned red_tail_leave(int type, int n, int slot, int slot_max, int ticket_arg, int nparams);
 template <class T>
 struct RedTail;
