@@ -1836,10 +1836,33 @@ bool run_res_bres(op_set rset, const op_arg *ra, op_set bset, const op_arg *ba,
                           : res_bres_t<float>(rset, ra, bset, ba);
 }
 
+// res_calc's arguments in the airfoil shape: both x through one dim-2 map
+// (idx 0, 1), q and adt through another, one dataset each, sizes that keep
+// 32-bit index arithmetic
+static bool flux_pair_shape(const op_arg *ra, size_t nval) {
+  auto pair = [](const op_arg &a, const op_arg &b) {
+    return a.map && a.map == b.map && a.map->dim == 2 && a.idx == 0 && b.idx == 1;
+  };
+  return pair(ra[0], ra[1]) && pair(ra[2], ra[3]) && pair(ra[4], ra[5]) &&
+         ra[2].map == ra[4].map && ra[0].dat == ra[1].dat && ra[2].dat == ra[3].dat &&
+         ra[4].dat == ra[5].dat && (long long)nval < (1LL << 30) &&
+         (long long)ra[2].dat->set->size < (1LL << 30) &&
+         (long long)ra[0].dat->set->size < (1LL << 30);
+}
+
+// the order the flux pass takes these edges in; nullptr: the loop's own
+static const SlotPlan::Order *flux_order(SlotPlan *sp, const op_arg *ra) {
+  if (!tuning("flux_order", 1) || !tuning("flux_pair", 1) ||
+      !flux_pair_shape(ra, (size_t)sp->na + sp->nb + 1))
+    return nullptr;
+  return get_flux_order(sp, ra[0].map, ra[2].map);
+}
+
 // the flux pass of res_calc (and bres_calc's values when B.n > 0) into vals
 template <class T>
-static void launch_flux(const op_arg *ra, const ResEdges<T> &E, const BresEdges<T> &B, T *vals,
-                        size_t nval, const AirConsts<T> &K, cudaStream_t s) {
+static void launch_flux(SlotPlan *sp, const op_arg *ra, const ResEdges<T> &E,
+                        const BresEdges<T> &B, T *vals, size_t nval, const AirConsts<T> &K,
+                        cudaStream_t s) {
   const long long nflux = (long long)E.n + B.n;
   // flux_ctas_per_sm = 0: one edge per thread (many short CTAs balance the
   // SMs); n > 0: at most n CTAs per SM, grid-stride (default 16 in FP32,
@@ -1848,25 +1871,18 @@ static void launch_flux(const op_arg *ra, const ResEdges<T> &E, const BresEdges<
   long long fg = (nflux + 255) / 256;
   if (per_sm > 0) fg = std::min(fg, (long long)rt().num_sms * per_sm);
   const unsigned fgrid = (unsigned)std::max(1LL, fg);
-  auto pair = [](const op_arg &a, const op_arg &b) {
-    return a.map && a.map == b.map && a.map->dim == 2 && a.idx == 0 && b.idx == 1;
-  };
-  const bool shape = pair(ra[0], ra[1]) && pair(ra[2], ra[3]) && pair(ra[4], ra[5]) &&
-                     ra[2].map == ra[4].map && ra[0].dat == ra[1].dat && ra[2].dat == ra[3].dat &&
-                     ra[4].dat == ra[5].dat && (long long)nval < (1LL << 30) &&
-                     (long long)ra[2].dat->set->size < (1LL << 30) &&
-                     (long long)ra[0].dat->set->size < (1LL << 30);
-  if (shape && tuning("flux_pair", 1)) {
+  if (flux_pair_shape(ra, nval) && tuning("flux_pair", 1)) {
+    const SlotPlan::Order *o = flux_order(sp, ra);
+    const int2 *pe = o ? o->d_edge : reinterpret_cast<const int2 *>(map_dev(ra[0].map));
+    const int2 *pc = o ? o->d_cell : reinterpret_cast<const int2 *>(map_dev(ra[2].map));
     const RedTail<T> tail = red_tail_take<T>();
-    launch_pdl(k_res_flux_pair<T>, fgrid + (tail.n ? 1 : 0), 256, 0, s, E.n,
-               reinterpret_cast<const int2 *>(map_dev(ra[0].map)),
-               reinterpret_cast<const int2 *>(map_dev(ra[2].map)), E.xa, E.qa, E.adta, B, vals, K,
-               tail);
-  }
-  else if (tuning("flux_pipe", 0))
+    launch_pdl(k_res_flux_pair<T>, fgrid + (tail.n ? 1 : 0), 256, 0, s, E.n, pe, pc, E.xa, E.qa,
+               E.adta, B, vals, K, tail);
+  } else if (tuning("flux_pipe", 0)) {
     launch_pdl(k_res_flux_list<T, true, sizeof(T) == 4 ? 6 : 3>, fgrid, 256, 0, s, E, B, vals, K);
-  else
+  } else {
     launch_pdl(k_res_flux_list<T, false, sizeof(T) == 4 ? 8 : 4>, fgrid, 256, 0, s, E, B, vals, K);
+  }
 }
 
 // the persistent chain's queue for a slot plan (host side of ChainSchedDev)
@@ -1977,20 +1993,6 @@ static ChainSched *chain_sched(SlotPlan *sp, int et, int ct, int lag) {
   return cs;
 }
 
-// res_calc's arguments in the airfoil shape: both x through one dim-2 map
-// (idx 0, 1), q and adt through another, one dataset each, sizes that keep
-// 32-bit index arithmetic
-static bool flux_pair_shape(const op_arg *ra, size_t nval) {
-  auto pair = [](const op_arg &a, const op_arg &b) {
-    return a.map && a.map == b.map && a.map->dim == 2 && a.idx == 0 && b.idx == 1;
-  };
-  return pair(ra[0], ra[1]) && pair(ra[2], ra[3]) && pair(ra[4], ra[5]) &&
-         ra[2].map == ra[4].map && ra[0].dat == ra[1].dat && ra[2].dat == ra[3].dat &&
-         ra[4].dat == ra[5].dat && (long long)nval < (1LL << 30) &&
-         (long long)ra[2].dat->set->size < (1LL << 30) &&
-         (long long)ra[0].dat->set->size < (1LL << 30);
-}
-
 // the plans and value buffer of a res_calc (+ bres_calc) chain; nullptr
 // when the mesh does not suit slots; *err when a plan failed
 template <class T>
@@ -2035,12 +2037,13 @@ static SlotPlan *chain_plans(op_set rset, const op_arg *ra, op_set bset, const o
 // contributions and for bres_calc on its own.
 bool coloured_fold() { return tuning("coloured_fold", 1) && tuning("gather_slots", 1); }
 
-static const int *coloured_ell(SlotPlan *sp, op_set rset, const op_arg *ra, op_set bset,
-                               const op_arg *ba, const ColourKey &key) {
+static const int *coloured_ell(SlotPlan *sp, const SlotPlan::Order *o, op_set rset,
+                               const op_arg *ra, op_set bset, const op_arg *ba,
+                               const ColourKey &key) {
   DevPlan *p = get_plan(key.rname, rset, key.rpart, 8, ra, 4, kResInds);
   DevPlan *pb = ba ? get_plan(key.bname, bset, key.bpart, 6, ba, 4, kBresInds) : nullptr;
   if (!p || (ba && !pb)) return nullptr;
-  return get_coloured_lists(sp, p, key.rblock > 0 ? key.rblock : 512, pb,
+  return get_coloured_lists(sp, o, p, key.rblock > 0 ? key.rblock : 512, pb,
                             key.bblock > 0 ? key.bblock : 512);
 }
 
@@ -2082,7 +2085,7 @@ static bool res_flux_ahead_t(op_set rset, const op_arg *ra, op_set bset, const o
   if (ra[4].dat == adt) E.adta = (const T *)adt_now;
   if (ra[5].dat == adt) E.adtb = (const T *)adt_now;
   if (ba && ba[3].dat == adt) B.adt = (const T *)adt_now;
-  launch_flux<T>(ra, E, B, (T *)sp->d_buf, (size_t)sp->na + sp->nb + 1, K, rt().stream);
+  launch_flux<T>(sp, ra, E, B, (T *)sp->d_buf, (size_t)sp->na + sp->nb + 1, K, rt().stream);
   return true;
 }
 
@@ -2675,10 +2678,13 @@ static bool res_chain_t(char const *loop_name, op_set rset, const op_arg *ra, op
   const size_t nval = (size_t)sp->na + sp->nb + 1;
   T *vals = (T *)sp->d_buf;
   const bool col = effective_strategy(key.rname) == OP2B_STRATEGY_COLOURED;
-  const int *ell = sp->d_ell;
+  // the lists that go with the flux pass's order
+  const SlotPlan::Order *order = flux_order(sp, ra);
+  if (error_pending()) return true;
+  const int *ell = order ? order->d_ell : sp->d_ell;
   if (col) {
     if (!coloured_fold()) return false;
-    ell = coloured_ell(sp, rset, ra, bset, ba, key);
+    ell = coloured_ell(sp, order, rset, ra, bset, ba, key);
     if (error_pending()) return true;
     if (!ell) return false;
   }
@@ -2708,7 +2714,7 @@ static bool res_chain_t(char const *loop_name, op_set rset, const op_arg *ra, op
       goto chained;
     if (!flux_done) {
       PhaseScope ph(name + ":flux");
-      launch_flux<T>(ra, E, B, vals, nval, K, s);
+      launch_flux<T>(sp, ra, E, B, vals, nval, K, s);
     }
     {
     PhaseScope ph(name + ":fold");

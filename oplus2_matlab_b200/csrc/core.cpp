@@ -95,6 +95,7 @@ int op2b_set_reduction(int m) {
 int op2b_set_tuning(const char *key, int value) {
   flush_pending();
   if (!key) return -1;
+  ahead_drop();  // values run ahead may be laid out for another setting
   int old = tuning(key, -1);
   rt().tuning[key] = value;
   return old;

@@ -92,8 +92,16 @@ struct SlotPlan {
   size_t buf_bytes = 0;
   ChainSched *chain = nullptr;  // built by the first persistent chain launch
   bool chain_unsuited = false;  // a cell tile reads too many flux tiles for it
+  // the edges of a in the order the flux pass takes them (get_flux_order)
+  struct Order {
+    op_map mx, mq;          // the maps of the edges' nodes and cells
+    int2 *d_edge, *d_cell;  // [na] the edges' rows of them
+    int *d_ell;             // the lists, with the places of the edges' values
+  };
+  std::vector<std::unique_ptr<Order>> orders;
   struct Coloured {  // get_coloured_lists
     const DevPlan *p, *pb;
+    const Order *o;
     int nt, nbt, *d_ell;
   };
   std::vector<Coloured> coloured;
@@ -108,8 +116,15 @@ void release_tile_plan(SlotPlan *sp);
 // threads per block) and b (pb, nbt; nullable): by block colour, then by
 // strip of nt elements of the block, thread colour and slot, b's after a's;
 // entry index << 2 | last of its block << 1 | negate, -1 past the end.
+// o: when the flux pass has an order of its own.
 // Device memory kept with the slot plan; nullptr when the indices do not fit.
-const int *get_coloured_lists(SlotPlan *sp, const DevPlan *p, int nt, const DevPlan *pb, int nbt);
+const int *get_coloured_lists(SlotPlan *sp, const SlotPlan::Order *o, const DevPlan *p, int nt,
+                              const DevPlan *pb, int nbt);
+
+// Find or build the flux pass's order of a's edges, whose nodes and cells are
+// columns 0 and 1 of the dim-2 maps mx and mq; nullptr during a capture that
+// comes before it is built.
+const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq);
 
 // widest list the fold kernels accept
 constexpr int kMaxSlotWidth = 8;

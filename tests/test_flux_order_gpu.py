@@ -1,0 +1,52 @@
+"""The flux pass's own order of the edges (knob flux_order) against the loop's:
+every field bit for bit, over sizes around a chunk of 1024 edges, numberings
+with and without locality, both precisions, GATHER and COLOURED, the residual
+alone and the fused chain; and the knob changed between two loops whose flux
+pass has run ahead."""
+import numpy as np
+import pytest
+
+from oplus2_matlab_b200 import api, apps
+from oplus2_matlab_b200 import mesh as M
+
+pytestmark = pytest.mark.gpu
+
+
+def solve(mesh, dt, strategy, order, flip=False):
+    api.set_error_mode(api.ERRORS_RETURN)
+    api.op_init([], 0)
+    lib = api.lib()
+    old = api.set_strategy(strategy)
+    api.set_reduction(api.REDUCE_TREE)
+    lib.op2b_set_tuning(b"flux_order", order)
+    try:
+        A = apps.Airfoil(mesh, dt)
+        for nm in ("adt_calc", "res_calc", "bres_calc"):
+            A.loop(nm)
+        api.sync()
+        rms = list(A.iterate(3))
+        if flip:
+            lib.op2b_set_tuning(b"flux_order", 1 - order)
+        rms += list(A.iterate(2))
+        st = {k: v.copy() for k, v in A.fetch().items()}
+        assert api.last_error() == ""
+        return st, rms
+    finally:
+        lib.op2b_set_tuning(b"flux_order", 1)
+        api.set_strategy(old)
+        api.op_exit()
+        api.clear_error()
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("I,J,scramble", [(2, 4, False), (17, 10, False), (19, 9, False), (40, 60, False),
+                                          (60, 90, True), (131, 77, False)])
+def test_same_fields(dt, I, J, scramble):
+    mesh = M.naca0012(I, J, scramble=scramble)
+    for strategy in (api.STRATEGY_GATHER, api.STRATEGY_COLOURED):
+        a, ra = solve(mesh, dt, strategy, 0)
+        b, rb = solve(mesh, dt, strategy, 1)
+        c, rc = solve(mesh, dt, strategy, 1, flip=True)
+        for k in a:
+            assert a[k].tobytes() == b[k].tobytes() == c[k].tobytes(), (strategy, k)
+        assert ra == rb == rc
