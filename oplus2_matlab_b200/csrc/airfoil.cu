@@ -1855,7 +1855,7 @@ static const SlotPlan::Order *flux_order(SlotPlan *sp, const op_arg *ra) {
   if (!tuning("flux_order", 1) || !tuning("flux_pair", 1) ||
       !flux_pair_shape(ra, (size_t)sp->na + sp->nb + 1))
     return nullptr;
-  return get_flux_order(sp, ra[0].map, ra[2].map);
+  return get_flux_order(sp, ra[0].map, ra[2].map, ra[0].dat);
 }
 
 // the flux pass of res_calc (and bres_calc's values when B.n > 0) into vals

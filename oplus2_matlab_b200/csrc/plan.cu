@@ -1850,7 +1850,139 @@ __global__ void k_order_lists(size_t n, int na, const int *__restrict__ ell,
   }
 }
 
-const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq) {
+// A numbering without locality makes every gather of the pass a sector of its
+// own: 192 bytes an edge besides its 32, and each cell and node fetched for
+// every edge it is on.  The nodes' coordinates then order all edges: strips of
+// equal numbers of edges along the first coordinate, each by the second, so
+// that a CTA's edges share cells and nodes, which L1 keeps.  (Coordinates are a
+// guess -- res_calc's first dataset, two reals per node -- and the order is
+// dropped when a sample of it is no better.)  A counting sort: the strips by a
+// histogram of the first coordinate in 65,536 steps, then one bin per strip
+// and step of the second.  Edges of one bin lie in any order; the sums do not
+// depend on it.
+constexpr int kCoordSteps = 65536;
+
+// distinct lines of 8 cells among the first cells of a chunk's edges
+__global__ void __launch_bounds__(kOrderChunk)
+    k_chunk_lines(int step, int na, const int2 *__restrict__ cell, unsigned long long *lines) {
+  __shared__ int key[kOrderChunk];
+  const int t = threadIdx.x, e = blockIdx.x * step * kOrderChunk + t;
+  key[t] = e < na ? cell[e].x >> 3 : INT_MAX;
+  __syncthreads();
+  bitonic_sort(key, kOrderChunk);
+  const int n = __syncthreads_count(key[t] != INT_MAX && (t == 0 || key[t] != key[t - 1]));
+  if (t == 0) atomicAdd(lines, (unsigned long long)n);
+}
+
+// distinct cells on a chunk's edges
+__global__ void __launch_bounds__(kOrderChunk)
+    k_chunk_cells(int step, int na, const int2 *__restrict__ cell, unsigned long long *cells) {
+  __shared__ int key[2 * kOrderChunk];
+  const int t = threadIdx.x, e = blockIdx.x * step * kOrderChunk + t;
+  key[t] = e < na ? cell[e].x : INT_MAX;
+  key[t + kOrderChunk] = e < na ? cell[e].y : INT_MAX;
+  __syncthreads();
+  bitonic_sort(key, 2 * kOrderChunk);
+  int n = 0;
+  for (int i = t; i < 2 * kOrderChunk; i += kOrderChunk)
+    n += __syncthreads_count(key[i] != INT_MAX && (i == 0 || key[i] != key[i - 1]));
+  if (t == 0) atomicAdd(cells, (unsigned long long)n);
+}
+
+// an order of floats as unsigned integers; what is not finite counts as 0
+__device__ __forceinline__ unsigned coord_key(float f) {
+  const unsigned u = __float_as_uint(isfinite(f) ? f : 0.0f);
+  return u >> 31 ? ~u : u | 0x80000000u;
+}
+__device__ __forceinline__ float coord_of(unsigned k) {
+  return __uint_as_float(k >> 31 ? k & 0x7fffffffu : ~k);
+}
+
+template <class T>
+__global__ void k_coord_bounds(int n, const T *__restrict__ x, unsigned *lo, unsigned *hi) {
+  unsigned a[2] = {~0u, ~0u}, b[2] = {0u, 0u};
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    for (int d = 0; d < 2; d++) {
+      const unsigned k = coord_key((float)x[2 * (size_t)i + d]);
+      a[d] = min(a[d], k);
+      b[d] = max(b[d], k);
+    }
+  for (int d = 0; d < 2; d++) {
+    a[d] = __reduce_min_sync(0xffffffffu, a[d]);
+    b[d] = __reduce_max_sync(0xffffffffu, b[d]);
+    if ((threadIdx.x & 31) == 0) {
+      atomicMin(lo + d, a[d]);
+      atomicMax(hi + d, b[d]);
+    }
+  }
+}
+
+template <class T>
+__device__ __forceinline__ int coord_step(const T *x, int node, int d, const unsigned *lo,
+                                          const unsigned *hi) {
+  const float l = coord_of(lo[d]), h = coord_of(hi[d]);
+  const float f = coord_of(coord_key((float)x[2 * (size_t)node + d]));
+  const float s = h > l ? (f - l) / (h - l) * kCoordSteps : 0.0f;
+  return max(0, min(kCoordSteps - 1, (int)s));
+}
+
+template <class T>
+__global__ void k_strip_hist(int na, const int2 *__restrict__ edge, const T *__restrict__ x,
+                             const unsigned *lo, const unsigned *hi, int *hist) {
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < na; e += gridDim.x * blockDim.x)
+    atomicAdd(hist + coord_step(x, edge[e].x, 0, lo, hi), 1);
+}
+
+// before[s]: edges whose first coordinate lies in an earlier step than s
+template <class T>
+__global__ void k_bin_hist(int na, int nstrip, const int2 *__restrict__ edge,
+                           const T *__restrict__ x, const unsigned *lo, const unsigned *hi,
+                           const int *__restrict__ before, int *__restrict__ key, int *bins) {
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < na; e += gridDim.x * blockDim.x) {
+    const int node = edge[e].x;
+    const int strip = (int)((long long)before[coord_step(x, node, 0, lo, hi)] * nstrip / na);
+    key[e] = strip * kCoordSteps + coord_step(x, node, 1, lo, hi);
+    atomicAdd(bins + key[e], 1);
+  }
+}
+
+__global__ void k_bin_place(int na, const int2 *__restrict__ edge, const int2 *__restrict__ cell,
+                            const int *__restrict__ key, int *bins, int2 *__restrict__ edge_out,
+                            int2 *__restrict__ cell_out, int *__restrict__ pos) {
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < na; e += gridDim.x * blockDim.x) {
+    const int p = atomicAdd(bins + key[e], 1);
+    edge_out[p] = edge[e];
+    cell_out[p] = cell[e];
+    pos[e] = p;
+  }
+}
+
+// the coordinate order of all edges into edge_out, cell_out and pos (queued)
+template <class T>
+static bool coord_order(int na, int nnode, const int2 *edge, const int2 *cell, const T *x,
+                        int2 *edge_out, int2 *cell_out, int *pos, cudaStream_t s) {
+  int nstrip = 1;
+  while ((long long)(nstrip + 1) * (nstrip + 1) * kOrderChunk <= na && nstrip < 1024) nstrip++;
+  const size_t nbin = (size_t)nstrip * kCoordSteps;
+  int *mem = nullptr;  // bounds (lo 2, hi 2) | first coordinate's histogram | bins | keys
+  const size_t words = 4 + kCoordSteps + nbin + (size_t)na;
+  if (pool_malloc_async((void **)&mem, sizeof(int) * words, s) != cudaSuccess) return false;
+  unsigned *lo = (unsigned *)mem, *hi = lo + 2;
+  int *hist = mem + 4, *bins = hist + kCoordSteps, *key = bins + nbin;
+  OP2B_CUDA(cudaMemsetAsync(lo, 0xff, 2 * sizeof(int), s));
+  OP2B_CUDA(cudaMemsetAsync(hi, 0, sizeof(int) * (2 + kCoordSteps + nbin), s));
+  const int grid = rt().num_sms * 8;
+  k_coord_bounds<T><<<grid, 256, 0, s>>>(nnode, x, lo, hi);
+  k_strip_hist<T><<<grid, 256, 0, s>>>(na, edge, x, lo, hi, hist);
+  exclusive_scan_nosync(hist, hist, kCoordSteps, s);
+  k_bin_hist<T><<<grid, 256, 0, s>>>(na, nstrip, edge, x, lo, hi, hist, key, bins);
+  exclusive_scan_nosync(bins, bins, (int)nbin, s);
+  k_bin_place<<<grid, 256, 0, s>>>(na, edge, cell, key, bins, edge_out, cell_out, pos);
+  OP2B_CUDA(cudaFreeAsync(mem, s));
+  return true;
+}
+
+const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq, op_dat x) {
   for (auto &o : sp->orders)
     if (o->mx == mx && o->mq == mq) return o->d_edge ? o.get() : nullptr;
   cudaStream_t s = rt().stream;
@@ -1868,7 +2000,7 @@ const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq) {
   o->d_ell = nullptr;
   // what it would give, from at most 128 chunks: a twentieth fewer lines at
   // least, or the loop's own maps do (and a scrambled mesh pays no memory)
-  unsigned long long *cost = nullptr, h[2] = {0, 0};
+  unsigned long long *cost = nullptr, h[3] = {0, 0, 0};
   int *pos = nullptr;
   if (pool_malloc_async((void **)&cost, sizeof h, s) != cudaSuccess) {
     cudaGetLastError();
@@ -1876,19 +2008,43 @@ const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq) {
   }
   OP2B_CUDA(cudaMemsetAsync(cost, 0, sizeof h, s));
   const int step = (nchunk + 127) / 128;
-  k_flux_order<<<(nchunk + step - 1) / step, kOrderChunk, 0, s>>>(step, na, edge, cell, nullptr,
-                                                                  nullptr, nullptr, cost);
+  const int nsample = (nchunk + step - 1) / step;
+  k_flux_order<<<nsample, kOrderChunk, 0, s>>>(step, na, edge, cell, nullptr, nullptr, nullptr,
+                                               cost);
+  k_chunk_lines<<<nsample, kOrderChunk, 0, s>>>(step, na, cell, cost + 2);
   OP2B_CUDA(cudaMemcpyAsync(h, cost, sizeof h, cudaMemcpyDeviceToHost, s));
-  OP2B_CUDA(cudaFreeAsync(cost, s));
   OP2B_CUDA(cudaStreamSynchronize(s));
-  if ((double)h[1] <= 0.95 * (double)h[0] &&
+  // half as many lines as edges or more: no locality (a mesh numbered along
+  // its rows has 70 to 130 lines per 1024 edges, one with a good order fewer
+  // than 200)
+  const bool scattered = h[2] * 2 > (unsigned long long)nsample * kOrderChunk;
+  const bool lines = !scattered && (double)h[1] <= 0.95 * (double)h[0];
+  if ((lines || scattered) &&
       pool_malloc_async((void **)&pos, sizeof(int) * (size_t)na, s) == cudaSuccess) {
     o->d_edge = (int2 *)dev_alloc(sizeof(int2) * (size_t)na);
     o->d_cell = (int2 *)dev_alloc(sizeof(int2) * (size_t)na);
     o->d_ell = (int *)dev_alloc(sizeof(int) * nlist);
-    if (o->d_edge && o->d_cell && o->d_ell) {
+    bool good = o->d_edge && o->d_cell && o->d_ell;
+    if (good && lines) {
       k_flux_order<<<nchunk, kOrderChunk, 0, s>>>(1, na, edge, cell, o->d_edge, o->d_cell, pos,
                                                   nullptr);
+    } else if (good) {
+      const int nnode = x->set->size;
+      good = strcmp(x->type, "double") == 0
+                 ? coord_order(na, nnode, edge, cell, (const double *)x->data_d, o->d_edge,
+                               o->d_cell, pos, s)
+                 : coord_order(na, nnode, edge, cell, (const float *)x->data_d, o->d_edge,
+                               o->d_cell, pos, s);
+      // the same sample of the new order: distinct cells of its edges instead
+      // of lines (the cells' numbers stay scattered)
+      OP2B_CUDA(cudaMemsetAsync(cost, 0, sizeof h, s));
+      if (good) k_chunk_cells<<<nsample, kOrderChunk, 0, s>>>(step, na, o->d_cell, cost);
+      if (good) k_chunk_cells<<<nsample, kOrderChunk, 0, s>>>(step, na, cell, cost + 1);
+      OP2B_CUDA(cudaMemcpyAsync(h, cost, sizeof h, cudaMemcpyDeviceToHost, s));
+      OP2B_CUDA(cudaStreamSynchronize(s));
+      good = good && (double)h[0] < 0.75 * (double)h[1];
+    }
+    if (good) {
       k_order_lists<<<rt().num_sms * 8, 256, 0, s>>>(nlist, na, sp->d_ell, pos, o->d_ell);
     } else {
       dev_free(o->d_edge);
@@ -1898,6 +2054,7 @@ const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq) {
     }
     OP2B_CUDA(cudaFreeAsync(pos, s));
   }
+  OP2B_CUDA(cudaFreeAsync(cost, s));
   cudaGetLastError();
   sp->orders.push_back(std::move(o));
   return sp->orders.back()->d_edge ? sp->orders.back().get() : nullptr;

@@ -122,9 +122,10 @@ const int *get_coloured_lists(SlotPlan *sp, const SlotPlan::Order *o, const DevP
                               const DevPlan *pb, int nbt);
 
 // Find or build the flux pass's order of a's edges, whose nodes and cells are
-// columns 0 and 1 of the dim-2 maps mx and mq; nullptr during a capture that
-// comes before it is built.
-const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq);
+// columns 0 and 1 of the dim-2 maps mx and mq and whose nodes have the dataset
+// x (two reals: taken for coordinates when the numbering has no locality);
+// nullptr: the loop's own order, or a capture that comes before it is built.
+const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq, op_dat x);
 
 // widest list the fold kernels accept
 constexpr int kMaxSlotWidth = 8;
