@@ -159,18 +159,7 @@ __device__ __forceinline__ void list_head(const int *__restrict__ ell, int W, in
   }
 }
 
-template <class T>
-__device__ __forceinline__ void add_listed(T r[4], int k, const T f[4]) {
-  if (k < 0) return;
-  if (k & 1) {
-    r[0] -= f[0]; r[1] -= f[1]; r[2] -= f[2]; r[3] -= f[3];
-  } else {
-    r[0] += f[0]; r[1] += f[1]; r[2] += f[2]; r[3] += f[3];
-  }
-}
-
-// the same without a branch, for an entry that is there: r + f or r + (-f), as
-// one rounding of (+-1) f + r
+// +-1 by the entry's lowest bit; r + f and r - f are one rounding of (+-1) f + r
 __device__ __forceinline__ float signed_one(int k, float) {
   return __int_as_float(0x3f800000 | k << 31);
 }
@@ -179,11 +168,18 @@ __device__ __forceinline__ double signed_one(int k, double) {
 }
 __device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+// r + f or r - f for an entry that is there
 template <class T>
 __device__ __forceinline__ void add_signed(T r[4], int k, const T f[4]) {
   const T s = signed_one(k, T(0));
 #pragma unroll
   for (int d = 0; d < 4; d++) r[d] = fma_rn(s, f[d], r[d]);
+}
+
+// the same; -1: no entry
+template <class T>
+__device__ __forceinline__ void add_listed(T r[4], int k, const T f[4]) {
+  if (k >= 0) add_signed(r, k, f);
 }
 
 // the same for a list in the order of the two-level colouring (entry = index

@@ -1742,17 +1742,17 @@ const int *get_coloured_lists(SlotPlan *sp, const SlotPlan::Order *o, const DevP
 
 // ------------------------------------------------------------ flux order --
 // The flux pass reads its edges' cells and nodes through L1, a warp's 32 edges
-// at a time, and an edge loop's own order makes that expensive: a mesh
-// generator emits an edge to the next cell of a row, then one to the next row,
-// so the lanes of one load alternate between distant lines and L1 serves half
-// as much per cycle as it could.  Inside chunks of kOrderChunk edges the pass
+// at a time, and an edge loop's own order makes that dearer than it need be: a
+// mesh generator emits an edge to the next cell of a row, then one to the next
+// row, so the lanes of one load alternate between distant lines.  Inside chunks of kOrderChunk edges the pass
 // therefore takes the edges sorted by the distance between their cells, then
 // by the first: runs of edges that step through both cells together.  A chunk
 // whose loads would not touch fewer lines so (a numbering without such
 // distances) keeps its order.  The values lie in v in the pass's order and the
 // lists say where: every cell still adds the same values in the same order.
-// Lines touched per warp of the NACA mesh: about half.  A captured iteration
-// at 407k FP64 cells, where L1 was the bound (78% busy): 46.5 -> 44.2 us; at 720k
+// Lines a warp's gathers touch on the NACA mesh: a tenth fewer (the run of 8
+// cells a line holds seldom starts on one).  A captured iteration at 407k FP64
+// cells, where L1 was the bound (78% busy): 46.5 -> 44.2 us; at 720k
 // FP32 39.8 either way (issue-bound), at 7k 7.7 -> 7.45.
 constexpr int kOrderChunk = 1024;
 
