@@ -411,9 +411,12 @@ __global__ void __launch_bounds__(256, MINB)
 // another (pecell), one dataset each -- one 8-byte load per map, 32-bit
 // index arithmetic (map values are checked against the target set's size
 // at op_decl_map; the host takes this path only for sets below 2^30).
-template <class T>
+// ROWS: the edges' rows of both maps together, in an order of the pass's own
+// (SlotPlan::Order); else the two maps in edge order
+template <class T, bool ROWS>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 4)
-    k_res_flux_pair(int ne, const int2 *__restrict__ pedge, const int2 *__restrict__ pecell,
+    k_res_flux_pair(int ne, const int4 *__restrict__ rows, const int2 *__restrict__ pedge,
+                    const int2 *__restrict__ pecell,
                     const T *__restrict__ x, const T *__restrict__ q,
                     const T *__restrict__ adt, BresEdges<T> B, T *__restrict__ v,
                     AirConsts<T> K, RedTail<T> tail) {
@@ -432,10 +435,17 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 4)
   const unsigned i0 = cta * blockDim.x + threadIdx.x;
   const unsigned stride = ctas * blockDim.x;
   int2 nn = make_int2(0, 0), cc = make_int2(0, 0);
-  if (i0 < n_e) {  // map entries: read-only, fetched before the wait
-    nn = ld_stream(pedge + i0);
-    cc = ld_stream(pecell + i0);
-  }
+  auto maps = [&](unsigned i) {
+    if (ROWS) {
+      const int4 r = ld_stream(rows + i);
+      nn = make_int2(r.x, r.y);
+      cc = make_int2(r.z, r.w);
+    } else {
+      nn = ld_stream(pedge + i);
+      cc = ld_stream(pecell + i);
+    }
+  };
+  if (i0 < n_e) maps(i0);  // map entries: read-only, fetched before the wait
   pdl_wait();
   pdl_trigger();
   for (unsigned i = i0; i < total; i += stride) {
@@ -447,10 +457,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 4)
       ld2(x + 2u * (unsigned)nn.x, p);
       ld2(x + 2u * (unsigned)nn.y, s);
       const T d1 = __ldg(adt + (unsigned)cc.x), d2 = __ldg(adt + (unsigned)cc.y);
-      if (i + stride < n_e) {
-        nn = ld_stream(pedge + i + stride);
-        cc = ld_stream(pecell + i + stride);
-      }
+      if (i + stride < n_e) maps(i + stride);
       res_flux(p, s, q1, q2, d1, d2, K.gm1, K.eps, f);
     } else {
       const int b = (int)(i - n_e);
@@ -1873,11 +1880,12 @@ static void launch_flux(SlotPlan *sp, const op_arg *ra, const ResEdges<T> &E,
   const unsigned fgrid = (unsigned)std::max(1LL, fg);
   if (flux_pair_shape(ra, nval) && tuning("flux_pair", 1)) {
     const SlotPlan::Order *o = flux_order(sp, ra);
-    const int2 *pe = o ? o->d_edge : reinterpret_cast<const int2 *>(map_dev(ra[0].map));
-    const int2 *pc = o ? o->d_cell : reinterpret_cast<const int2 *>(map_dev(ra[2].map));
     const RedTail<T> tail = red_tail_take<T>();
-    launch_pdl(k_res_flux_pair<T>, fgrid + (tail.n ? 1 : 0), 256, 0, s, E.n, pe, pc, E.xa, E.qa,
-               E.adta, B, vals, K, tail);
+    launch_pdl(o ? k_res_flux_pair<T, true> : k_res_flux_pair<T, false>,
+               fgrid + (tail.n ? 1 : 0), 256, 0, s, E.n, (const int4 *)(o ? o->d_rows : nullptr),
+               reinterpret_cast<const int2 *>(map_dev(ra[0].map)),
+               reinterpret_cast<const int2 *>(map_dev(ra[2].map)), E.xa, E.qa, E.adta, B, vals, K,
+               tail);
   } else if (tuning("flux_pipe", 0)) {
     launch_pdl(k_res_flux_list<T, true, sizeof(T) == 4 ? 6 : 3>, fgrid, 256, 0, s, E, B, vals, K);
   } else {

@@ -769,18 +769,40 @@ __global__ void k_check_blocks(PlanParams pp, const int *blkmap, const int *offs
 
 // ------------------------------------------------------------------ scan --
 
-__global__ void k_scan_chunks(const int *in, int *out, int n, int *sums, int chunk) {
-  int c0 = blockIdx.x * chunk;
-  int run = 0;
-  for (int r = 0; r < chunk; r += blockDim.x) {
-    int i = c0 + r + threadIdx.x;
-    int v = (i < n && r + threadIdx.x < chunk) ? in[i] : 0;
-    int tot;
-    int x = block_excl_scan(v, &tot);
-    if (i < n && r + threadIdx.x < chunk) out[i] = run + x;
-    run += tot;
+// a chunk of kScanChunk values per CTA of 1024, eight consecutive ones per thread
+constexpr int kScanChunk = 8192;
+__global__ void __launch_bounds__(1024) k_scan_chunks(const int *in, int *out, int n, int *sums) {
+  const long long i0 = (long long)blockIdx.x * kScanChunk + threadIdx.x * 8;
+  int v[8], own = 0;
+  const bool whole = i0 + 8 <= n && ((uintptr_t)in & 15) == 0 && ((uintptr_t)out & 15) == 0;
+  if (whole) {
+    const int4 a = reinterpret_cast<const int4 *>(in + i0)[0];
+    const int4 b = reinterpret_cast<const int4 *>(in + i0)[1];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  } else {
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = i0 + k < n ? in[i0 + k] : 0;
   }
-  if (threadIdx.x == 0) sums[blockIdx.x] = run;
+#pragma unroll
+  for (int k = 0; k < 8; k++) own += v[k];
+  int total;
+  int run = block_excl_scan(own, &total);
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const int x = v[k];
+    v[k] = run;
+    run += x;
+  }
+  if (whole) {
+    reinterpret_cast<int4 *>(out + i0)[0] = make_int4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<int4 *>(out + i0)[1] = make_int4(v[4], v[5], v[6], v[7]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      if (i0 + k < n) out[i0 + k] = v[k];
+  }
+  if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
 __global__ void k_scan_add(int *out, int n, const int *offs, int chunk) {
@@ -793,12 +815,12 @@ __global__ void k_scan_add(int *out, int n, const int *offs, int chunk) {
 }
 
 void exclusive_scan_nosync(const int *d_in, int *d_out, int n, cudaStream_t s) {
-  const int chunk = 8192;
+  const int chunk = kScanChunk;
   const int nch = (n + chunk - 1) / chunk;
   if (n <= 0) return;
   int *sums = nullptr;
   OP2B_CUDA(pool_malloc_async((void **)&sums, sizeof(int) * (nch + 1), s));
-  k_scan_chunks<<<nch, 1024, 0, s>>>(d_in, d_out, n, sums, chunk);
+  k_scan_chunks<<<nch, 1024, 0, s>>>(d_in, d_out, n, sums);
   if (nch > 1) {
     exclusive_scan_nosync(sums, sums, nch, s);
     k_scan_add<<<nch, 1024, 0, s>>>(d_out, n, sums, chunk);
@@ -807,12 +829,12 @@ void exclusive_scan_nosync(const int *d_in, int *d_out, int n, cudaStream_t s) {
 }
 
 long long exclusive_scan(const int *d_in, int *d_out, int n, cudaStream_t s) {
-  const int chunk = 8192;
+  const int chunk = kScanChunk;
   int nch = (n + chunk - 1) / chunk;
   if (n <= 0) return 0;
   int *sums = nullptr;
   OP2B_CUDA(pool_malloc_async((void **)&sums, sizeof(int) * (nch + 1), s));
-  k_scan_chunks<<<nch, 1024, 0, s>>>(d_in, d_out, n, sums, chunk);
+  k_scan_chunks<<<nch, 1024, 0, s>>>(d_in, d_out, n, sums);
   if (nch > 1) {
     exclusive_scan(sums, sums, nch, s);
     k_scan_add<<<nch, 1024, 0, s>>>(d_out, n, sums, chunk);
@@ -1783,8 +1805,7 @@ __device__ __forceinline__ int order_cost(int t, int n, const int2 *e, const int
 // only the lines before and after are added up
 __global__ void __launch_bounds__(kOrderChunk)
     k_flux_order(int step, int na, const int2 *__restrict__ edge, const int2 *__restrict__ cell,
-                 int2 *__restrict__ edge_out, int2 *__restrict__ cell_out, int *__restrict__ pos,
-                 unsigned long long *cost) {
+                 int4 *__restrict__ rows, int *__restrict__ pos, unsigned long long *cost) {
   __shared__ unsigned long long key[kOrderChunk];
   __shared__ int2 e[kOrderChunk], c[kOrderChunk];
   __shared__ unsigned short at[kOrderChunk];
@@ -1835,8 +1856,7 @@ __global__ void __launch_bounds__(kOrderChunk)
   if (cost && t < 2) atomicAdd(cost + t, (unsigned long long)(t ? min(sum[0], sum[1]) : sum[0]));
   if (t >= n || !pos) return;
   const int i = sum[1] < sum[0] ? at[t] : t;
-  edge_out[e0 + t] = e[i];
-  cell_out[e0 + t] = c[i];
+  rows[e0 + t] = make_int4(e[i].x, e[i].y, c[i].x, c[i].y);
   pos[e0 + i] = e0 + t;
 }
 
@@ -1862,25 +1882,16 @@ __global__ void k_order_lists(size_t n, int na, const int *__restrict__ ell,
 // depend on it.
 constexpr int kCoordSteps = 65536;
 
-// distinct lines of 8 cells among the first cells of a chunk's edges
-__global__ void __launch_bounds__(kOrderChunk)
-    k_chunk_lines(int step, int na, const int2 *__restrict__ cell, unsigned long long *lines) {
-  __shared__ int key[kOrderChunk];
-  const int t = threadIdx.x, e = blockIdx.x * step * kOrderChunk + t;
-  key[t] = e < na ? cell[e].x >> 3 : INT_MAX;
-  __syncthreads();
-  bitonic_sort(key, kOrderChunk);
-  const int n = __syncthreads_count(key[t] != INT_MAX && (t == 0 || key[t] != key[t - 1]));
-  if (t == 0) atomicAdd(lines, (unsigned long long)n);
-}
-
 // distinct cells on a chunk's edges
 __global__ void __launch_bounds__(kOrderChunk)
-    k_chunk_cells(int step, int na, const int2 *__restrict__ cell, unsigned long long *cells) {
+    k_chunk_cells(int step, int na, const int2 *__restrict__ cell, const int4 *__restrict__ rows,
+                  unsigned long long *cells) {
   __shared__ int key[2 * kOrderChunk];
   const int t = threadIdx.x, e = blockIdx.x * step * kOrderChunk + t;
-  key[t] = e < na ? cell[e].x : INT_MAX;
-  key[t + kOrderChunk] = e < na ? cell[e].y : INT_MAX;
+  int2 c = make_int2(INT_MAX, INT_MAX);
+  if (e < na) c = cell ? cell[e] : make_int2(rows[e].z, rows[e].w);
+  key[t] = c.x;
+  key[t + kOrderChunk] = c.y;
   __syncthreads();
   bitonic_sort(key, 2 * kOrderChunk);
   int n = 0;
@@ -1926,65 +1937,70 @@ __device__ __forceinline__ int coord_step(const T *x, int node, int d, const uns
   return max(0, min(kCoordSteps - 1, (int)s));
 }
 
+// steps[e]: both coordinates' steps of the edge's first node
 template <class T>
 __global__ void k_strip_hist(int na, const int2 *__restrict__ edge, const T *__restrict__ x,
-                             const unsigned *lo, const unsigned *hi, int *hist) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < na; e += gridDim.x * blockDim.x)
-    atomicAdd(hist + coord_step(x, edge[e].x, 0, lo, hi), 1);
+                             const unsigned *lo, const unsigned *hi, unsigned *__restrict__ steps,
+                             int *hist) {
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < na; e += gridDim.x * blockDim.x) {
+    const int node = edge[e].x, sx = coord_step(x, node, 0, lo, hi);
+    steps[e] = (unsigned)sx << 16 | (unsigned)coord_step(x, node, 1, lo, hi);
+    atomicAdd(hist + sx, 1);
+  }
 }
 
-// before[s]: edges whose first coordinate lies in an earlier step than s
-template <class T>
-__global__ void k_bin_hist(int na, int nstrip, const int2 *__restrict__ edge,
-                           const T *__restrict__ x, const unsigned *lo, const unsigned *hi,
-                           const int *__restrict__ before, int *__restrict__ key, int *bins) {
+// before[s]: edges whose first coordinate lies in an earlier step than s.  The
+// edge's bin takes the place of its steps
+__global__ void k_bin_hist(int na, int nstrip, const int *__restrict__ before, unsigned *steps,
+                           int *bins) {
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < na; e += gridDim.x * blockDim.x) {
-    const int node = edge[e].x;
-    const int strip = (int)((long long)before[coord_step(x, node, 0, lo, hi)] * nstrip / na);
-    key[e] = strip * kCoordSteps + coord_step(x, node, 1, lo, hi);
-    atomicAdd(bins + key[e], 1);
+    const unsigned s = steps[e];
+    const unsigned strip = (unsigned)((long long)before[s >> 16] * nstrip / na);
+    steps[e] = strip * kCoordSteps + (s & 0xffffu);
+    atomicAdd(bins + steps[e], 1);
   }
 }
 
 __global__ void k_bin_place(int na, const int2 *__restrict__ edge, const int2 *__restrict__ cell,
-                            const int *__restrict__ key, int *bins, int2 *__restrict__ edge_out,
-                            int2 *__restrict__ cell_out, int *__restrict__ pos) {
+                            const unsigned *__restrict__ bin, int *bins, int4 *__restrict__ rows,
+                            int *__restrict__ pos) {
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < na; e += gridDim.x * blockDim.x) {
-    const int p = atomicAdd(bins + key[e], 1);
-    edge_out[p] = edge[e];
-    cell_out[p] = cell[e];
+    const int p = atomicAdd(bins + bin[e], 1);
+    const int2 n = edge[e], c = cell[e];
+    rows[p] = make_int4(n.x, n.y, c.x, c.y);
     pos[e] = p;
   }
 }
 
-// the coordinate order of all edges into edge_out, cell_out and pos (queued)
+// the coordinate order of all edges into rows and pos (queued)
 template <class T>
 static bool coord_order(int na, int nnode, const int2 *edge, const int2 *cell, const T *x,
-                        int2 *edge_out, int2 *cell_out, int *pos, cudaStream_t s) {
+                        int4 *rows, int *pos, cudaStream_t s) {
   int nstrip = 1;
   while ((long long)(nstrip + 1) * (nstrip + 1) * kOrderChunk <= na && nstrip < 1024) nstrip++;
   const size_t nbin = (size_t)nstrip * kCoordSteps;
-  int *mem = nullptr;  // bounds (lo 2, hi 2) | first coordinate's histogram | bins | keys
+  int *mem = nullptr;  // bounds (lo 2, hi 2) | first coordinate's histogram | bins | steps
   const size_t words = 4 + kCoordSteps + nbin + (size_t)na;
   if (pool_malloc_async((void **)&mem, sizeof(int) * words, s) != cudaSuccess) return false;
   unsigned *lo = (unsigned *)mem, *hi = lo + 2;
-  int *hist = mem + 4, *bins = hist + kCoordSteps, *key = bins + nbin;
+  int *hist = mem + 4, *bins = hist + kCoordSteps;
+  unsigned *steps = (unsigned *)(bins + nbin);
   OP2B_CUDA(cudaMemsetAsync(lo, 0xff, 2 * sizeof(int), s));
   OP2B_CUDA(cudaMemsetAsync(hi, 0, sizeof(int) * (2 + kCoordSteps + nbin), s));
   const int grid = rt().num_sms * 8;
   k_coord_bounds<T><<<grid, 256, 0, s>>>(nnode, x, lo, hi);
-  k_strip_hist<T><<<grid, 256, 0, s>>>(na, edge, x, lo, hi, hist);
+  k_strip_hist<T><<<grid, 256, 0, s>>>(na, edge, x, lo, hi, steps, hist);
   exclusive_scan_nosync(hist, hist, kCoordSteps, s);
-  k_bin_hist<T><<<grid, 256, 0, s>>>(na, nstrip, edge, x, lo, hi, hist, key, bins);
+  k_bin_hist<<<grid, 256, 0, s>>>(na, nstrip, hist, steps, bins);
   exclusive_scan_nosync(bins, bins, (int)nbin, s);
-  k_bin_place<<<grid, 256, 0, s>>>(na, edge, cell, key, bins, edge_out, cell_out, pos);
+  k_bin_place<<<grid, 256, 0, s>>>(na, edge, cell, steps, bins, rows, pos);
   OP2B_CUDA(cudaFreeAsync(mem, s));
   return true;
 }
 
 const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq, op_dat x) {
   for (auto &o : sp->orders)
-    if (o->mx == mx && o->mq == mq) return o->d_edge ? o.get() : nullptr;
+    if (o->mx == mx && o->mq == mq) return o->d_rows ? o.get() : nullptr;
   cudaStream_t s = rt().stream;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   OP2B_CUDA(cudaStreamIsCapturing(s, &cap));
@@ -1996,50 +2012,44 @@ const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq, op_dat
   std::unique_ptr<SlotPlan::Order> o(new SlotPlan::Order());
   o->mx = mx;
   o->mq = mq;
-  o->d_edge = o->d_cell = nullptr;
+  o->d_rows = nullptr;
   o->d_ell = nullptr;
   // what it would give, from at most 128 chunks: a twentieth fewer lines at
-  // least, or the loop's own maps do (and a scrambled mesh pays no memory)
-  unsigned long long *cost = nullptr, h[3] = {0, 0, 0};
+  // least, or the loop's own maps do.  Three of a lane's four gathers on a line
+  // of its own: no locality (a mesh numbered along its rows has less than one)
+  unsigned long long *cost = nullptr, h[2] = {0, 0};
   int *pos = nullptr;
   if (pool_malloc_async((void **)&cost, sizeof h, s) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
+  const int step = (nchunk + 127) / 128, nsample = (nchunk + step - 1) / step;
   OP2B_CUDA(cudaMemsetAsync(cost, 0, sizeof h, s));
-  const int step = (nchunk + 127) / 128;
-  const int nsample = (nchunk + step - 1) / step;
-  k_flux_order<<<nsample, kOrderChunk, 0, s>>>(step, na, edge, cell, nullptr, nullptr, nullptr,
-                                               cost);
-  k_chunk_lines<<<nsample, kOrderChunk, 0, s>>>(step, na, cell, cost + 2);
+  k_flux_order<<<nsample, kOrderChunk, 0, s>>>(step, na, edge, cell, nullptr, nullptr, cost);
   OP2B_CUDA(cudaMemcpyAsync(h, cost, sizeof h, cudaMemcpyDeviceToHost, s));
   OP2B_CUDA(cudaStreamSynchronize(s));
-  // half as many lines as edges or more: no locality (a mesh numbered along
-  // its rows has 70 to 130 lines per 1024 edges, one with a good order fewer
-  // than 200)
-  const bool scattered = h[2] * 2 > (unsigned long long)nsample * kOrderChunk;
+  const long long sampled = std::min((long long)nsample * kOrderChunk, (long long)na);
+  const bool scattered = (long long)h[0] > 3 * sampled;
   const bool lines = !scattered && (double)h[1] <= 0.95 * (double)h[0];
   if ((lines || scattered) &&
       pool_malloc_async((void **)&pos, sizeof(int) * (size_t)na, s) == cudaSuccess) {
-    o->d_edge = (int2 *)dev_alloc(sizeof(int2) * (size_t)na);
-    o->d_cell = (int2 *)dev_alloc(sizeof(int2) * (size_t)na);
+    o->d_rows = (int4 *)dev_alloc(sizeof(int4) * (size_t)na);
     o->d_ell = (int *)dev_alloc(sizeof(int) * nlist);
-    bool good = o->d_edge && o->d_cell && o->d_ell;
+    bool good = o->d_rows && o->d_ell;
     if (good && lines) {
-      k_flux_order<<<nchunk, kOrderChunk, 0, s>>>(1, na, edge, cell, o->d_edge, o->d_cell, pos,
-                                                  nullptr);
+      k_flux_order<<<nchunk, kOrderChunk, 0, s>>>(1, na, edge, cell, o->d_rows, pos, nullptr);
     } else if (good) {
       const int nnode = x->set->size;
       good = strcmp(x->type, "double") == 0
-                 ? coord_order(na, nnode, edge, cell, (const double *)x->data_d, o->d_edge,
-                               o->d_cell, pos, s)
-                 : coord_order(na, nnode, edge, cell, (const float *)x->data_d, o->d_edge,
-                               o->d_cell, pos, s);
-      // the same sample of the new order: distinct cells of its edges instead
-      // of lines (the cells' numbers stay scattered)
+                 ? coord_order(na, nnode, edge, cell, (const double *)x->data_d, o->d_rows, pos, s)
+                 : coord_order(na, nnode, edge, cell, (const float *)x->data_d, o->d_rows, pos, s);
+      // a sample of the new order has a quarter fewer distinct cells than the
+      // old, or the coordinates were none
       OP2B_CUDA(cudaMemsetAsync(cost, 0, sizeof h, s));
-      if (good) k_chunk_cells<<<nsample, kOrderChunk, 0, s>>>(step, na, o->d_cell, cost);
-      if (good) k_chunk_cells<<<nsample, kOrderChunk, 0, s>>>(step, na, cell, cost + 1);
+      if (good) {
+        k_chunk_cells<<<nsample, kOrderChunk, 0, s>>>(step, na, nullptr, o->d_rows, cost);
+        k_chunk_cells<<<nsample, kOrderChunk, 0, s>>>(step, na, cell, nullptr, cost + 1);
+      }
       OP2B_CUDA(cudaMemcpyAsync(h, cost, sizeof h, cudaMemcpyDeviceToHost, s));
       OP2B_CUDA(cudaStreamSynchronize(s));
       good = good && (double)h[0] < 0.75 * (double)h[1];
@@ -2047,17 +2057,16 @@ const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq, op_dat
     if (good) {
       k_order_lists<<<rt().num_sms * 8, 256, 0, s>>>(nlist, na, sp->d_ell, pos, o->d_ell);
     } else {
-      dev_free(o->d_edge);
-      dev_free(o->d_cell);
+      dev_free(o->d_rows);
       dev_free(o->d_ell);
-      o->d_edge = nullptr;
+      o->d_rows = nullptr;
     }
     OP2B_CUDA(cudaFreeAsync(pos, s));
   }
   OP2B_CUDA(cudaFreeAsync(cost, s));
   cudaGetLastError();
   sp->orders.push_back(std::move(o));
-  return sp->orders.back()->d_edge ? sp->orders.back().get() : nullptr;
+  return sp->orders.back()->d_rows ? sp->orders.back().get() : nullptr;
 }
 
 }  // namespace op2b
@@ -2072,8 +2081,7 @@ void op2b_release_plans() {
     dev_free(up->d_buf);
     for (auto &c : up->coloured) dev_free(c.d_ell);
     for (auto &o : up->orders) {
-      dev_free(o->d_edge);
-      dev_free(o->d_cell);
+      dev_free(o->d_rows);
       dev_free(o->d_ell);
     }
   }

@@ -95,7 +95,7 @@ struct SlotPlan {
   // the edges of a in the order the flux pass takes them (get_flux_order)
   struct Order {
     op_map mx, mq;          // the maps of the edges' nodes and cells
-    int2 *d_edge, *d_cell;  // [na] the edges' rows of them
+    int4 *d_rows;           // [na] the edges' rows of them: two nodes, two cells
     int *d_ell;             // the lists, with the places of the edges' values
   };
   std::vector<std::unique_ptr<Order>> orders;
