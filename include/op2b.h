@@ -65,6 +65,9 @@ enum { OP2B_REDUCE_TREE = 0, OP2B_REDUCE_SEQ = 1 };
  *   "fold_cells"    1 (default): the per-cell pass of the airfoil shape (lists
  *                   of four, one x dataset) with every load of a thread's next
  *                   cell ahead of this cell's arithmetic; 0: the general pass
+ *   "flux_order"    1 (default): where the numbering has no locality, the flux
+ *                   pass takes the edges in the order of their nodes'
+ *                   coordinates; 0: in edge order
  *   "red_tail"      1 (default): the rms of an update is folded by the flux
  *                   pass behind it; 0: by the update's last block
  *   "coloured_fold" 1 (default): COLOURED res_calc [+ bres_calc ...] as the

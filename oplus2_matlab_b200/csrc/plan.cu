@@ -1650,6 +1650,23 @@ __global__ void k_fill_int(int *p, size_t n, int v) {
     p[i] = v;
 }
 
+// lines that the gathers of the two increments' targets touch (16-byte records,
+// eight lanes together) and that the lane before does not, in a sample of
+// chunks of kOrderChunk elements (chunks blockIdx.x * step)
+constexpr int kOrderChunk = 1024;
+__global__ void __launch_bounds__(kOrderChunk)
+    k_target_lines(int step, int n, SlotMaps sm, int *lines) {
+  const int t = threadIdx.x, e = blockIdx.x * step * kOrderChunk + t;
+  int k = 0;
+  if (e < n)
+    for (int s = 0; s < 2; s++) {
+      const int *m = sm.map[s] + sm.idx[s] + (size_t)e * sm.dim[s];
+      k += t % 8 == 0 || m[0] >> 3 != m[-sm.dim[s]] >> 3;
+    }
+  k = __reduce_add_sync(0xffffffffu, k);
+  if ((t & 31) == 0) atomicAdd(lines, k);
+}
+
 static std::vector<std::unique_ptr<SlotPlan>> g_slot_plans;
 
 SlotPlan *get_slot_plan(const GatherPlan *a, const GatherPlan *b) {
@@ -1668,15 +1685,28 @@ SlotPlan *get_slot_plan(const GatherPlan *a, const GatherPlan *b) {
     cudaStream_t s = rt().stream;
     const int grid = rt().num_sms * 8;
     int *cnt = nullptr;
-    OP2B_CUDA(pool_malloc_async((void **)&cnt, sizeof(int) * ((size_t)p.ntarget + 1), s));
-    int *mx = cnt + p.ntarget;
-    OP2B_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * ((size_t)p.ntarget + 1), s));
+    OP2B_CUDA(pool_malloc_async((void **)&cnt, sizeof(int) * ((size_t)p.ntarget + 2), s));
+    int *mx = cnt + p.ntarget;  // the longest list, the sample's lines
+    OP2B_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * ((size_t)p.ntarget + 2), s));
     k_ell_count<<<grid, 256, 0, s>>>(a->nactive, a->d_active, a->d_row, cnt);
     if (b && b->nactive) k_ell_count<<<grid, 256, 0, s>>>(b->nactive, b->d_active, b->d_row, cnt);
     k_max_int<<<grid, 256, 0, s>>>(cnt, p.ntarget, mx);
-    int w = 0;
-    OP2B_CUDA(cudaMemcpyAsync(&w, mx, sizeof(int), cudaMemcpyDeviceToHost, s));
+    // at most 128 chunks: three quarters of the targets on a line of their own is
+    // no locality (a mesh numbered along its rows has a quarter)
+    SlotMaps sm;
+    for (int i = 0; i < 2; i++) {
+      sm.map[i] = map_dev(a->maps[i]);
+      sm.dim[i] = a->maps[i]->dim;
+      sm.idx[i] = a->idxs[i];
+    }
+    const int nchunk = (p.na + kOrderChunk - 1) / kOrderChunk, step = (nchunk + 127) / 128;
+    const int nsample = (nchunk + step - 1) / step;
+    k_target_lines<<<nsample, kOrderChunk, 0, s>>>(step, p.na, sm, mx + 1);
+    int wl[2] = {0, 0};
+    OP2B_CUDA(cudaMemcpyAsync(wl, mx, sizeof wl, cudaMemcpyDeviceToHost, s));
     OP2B_CUDA(cudaStreamSynchronize(s));
+    const int w = wl[0];
+    p.scattered = 2LL * wl[1] > 3LL * std::min((long long)nsample * kOrderChunk, (long long)p.na);
     const long long nkeys = a->nkeys + (b ? b->nkeys : 0);
     if (w >= 1 && w <= kMaxSlotWidth && (long long)w * p.ntarget <= 2 * nkeys + p.ntarget) {
       p.width = w;
@@ -1763,102 +1793,25 @@ const int *get_coloured_lists(SlotPlan *sp, const SlotPlan::Order *o, const DevP
 }
 
 // ------------------------------------------------------------ flux order --
-// The flux pass reads its edges' cells and nodes through L1, a warp's 32 edges
-// at a time, and an edge loop's own order makes that dearer than it need be: a
-// mesh generator emits an edge to the next cell of a row, then one to the next
-// row, so the lanes of one load alternate between distant lines.  Inside chunks of kOrderChunk edges the pass
-// therefore takes the edges sorted by the distance between their cells, then
-// by the first: runs of edges that step through both cells together.  A chunk
-// whose loads would not touch fewer lines so (a numbering without such
-// distances) keeps its order.  The values lie in v in the pass's order and the
-// lists say where: every cell still adds the same values in the same order.
-// Lines a warp's gathers touch on the NACA mesh: a tenth fewer (the run of 8
-// cells a line holds seldom starts on one).  A captured iteration at 407k FP64
-// cells, where L1 was the bound (78% busy): 46.5 -> 44.2 us; at 720k
-// FP32 39.8 either way (issue-bound), at 7k 7.7 -> 7.45.
-constexpr int kOrderChunk = 1024;
-
-// lines a warp's loads of the edge at place t touch that the lane before it in
-// the same eighth (cells: 16-byte records) or quarter (nodes) does not
-__device__ __forceinline__ int order_cost(int t, int n, const int2 *e, const int2 *c,
-                                          const unsigned short *at) {
-  if (t >= n) return 0;
-  const int i = at[t];
-  const int2 ce = c[i], ne = e[i];
-  int k = 0;
-  if (t % 8 == 0) {
-    k = 2;
-  } else {
-    const int2 cp = c[at[t - 1]];
-    k = (ce.x >> 3 != cp.x >> 3) + (ce.y >> 3 != cp.y >> 3);
-  }
-  if (t % 16 == 0) {
-    k += 2;
-  } else {
-    const int2 np = e[at[t - 1]];
-    k += (ne.x >> 4 != np.x >> 4) + (ne.y >> 4 != np.y >> 4);
-  }
-  return k;
-}
-
-// chunks blockIdx.x * step, each into its part of the outputs; without them
-// only the lines before and after are added up
-__global__ void __launch_bounds__(kOrderChunk)
-    k_flux_order(int step, int na, const int2 *__restrict__ edge, const int2 *__restrict__ cell,
-                 int4 *__restrict__ rows, int *__restrict__ pos, unsigned long long *cost) {
-  __shared__ unsigned long long key[kOrderChunk];
-  __shared__ int2 e[kOrderChunk], c[kOrderChunk];
-  __shared__ unsigned short at[kOrderChunk];
-  const int t = threadIdx.x, e0 = blockIdx.x * step * kOrderChunk, n = min(kOrderChunk, na - e0);
-  key[t] = ~0ull;  // past the end: last
-  if (t < n) {
-    e[t] = edge[e0 + t];
-    c[t] = cell[e0 + t];
-    key[t] = (unsigned long long)((unsigned)(c[t].y - c[t].x) ^ 0x80000000u) << 32 |
-             (unsigned)c[t].x;
-  }
-  at[t] = (unsigned short)t;
-  __syncthreads();
-  int before = order_cost(t, n, e, c, at);
-  for (int k = 2; k <= kOrderChunk; k <<= 1)
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      if (t < kOrderChunk / 2) {
-        const int i = 2 * t - (t & (j - 1));
-        const unsigned long long a = key[i], b = key[i + j];
-        const unsigned short x = at[i], y = at[i + j];
-        // equal keys (two edges of the same cells) by edge, so the order is one
-        const bool gt = a > b || (a == b && x > y);
-        if (gt == ((i & k) == 0)) {
-          key[i] = b;
-          key[i + j] = a;
-          at[i] = y;
-          at[i + j] = x;
-        }
-      }
-      const int reach = j > 1 ? j >> 1 : k;
-      if (j > 32 || reach > 32) __syncthreads();
-      else __syncwarp();
-    }
-  __syncthreads();
-  int after = order_cost(t, n, e, c, at);
-  for (int o = 16; o > 0; o >>= 1) {
-    before += __shfl_xor_sync(0xffffffffu, before, o);
-    after += __shfl_xor_sync(0xffffffffu, after, o);
-  }
-  __shared__ int sum[2];
-  if (t < 2) sum[t] = 0;
-  __syncthreads();
-  if ((t & 31) == 0) {
-    atomicAdd(sum, before);
-    atomicAdd(sum + 1, after);
-  }
-  __syncthreads();
-  if (cost && t < 2) atomicAdd(cost + t, (unsigned long long)(t ? min(sum[0], sum[1]) : sum[0]));
-  if (t >= n || !pos) return;
-  const int i = sum[1] < sum[0] ? at[t] : t;
-  rows[e0 + t] = make_int4(e[i].x, e[i].y, c[i].x, c[i].y);
-  pos[e0 + i] = e0 + t;
-}
+// A numbering without locality makes every gather of the flux pass a sector of
+// its own: 192 bytes an edge besides its 32, and each cell and node fetched for
+// every edge it is on.  The nodes' coordinates then order the edges: strips of
+// equal numbers of edges along the first coordinate, each by the second, so
+// that a CTA's edges share cells and nodes, which L1 keeps.  The values lie in v
+// in the pass's order and the lists say where: every cell still adds the same
+// values in the same order.  (Coordinates are a guess -- res_calc's first
+// dataset, two reals per node -- and the order is dropped when a sample of it
+// is no better.)  A captured iteration of scrambled meshes: 720k FP32 cells 126 ->
+// 92 us, 2.88M 674 -> 471, 405k FP64 102 -> 81; the plan, about 0.5 ms of kernels
+// at 5.8M edges, is paid for by the first iterations.
+// A counting sort: the strips by a histogram of the first coordinate in 65,536
+// steps, then one bin per strip and step of the second.  Edges of one bin lie in
+// any order; the sums do not depend on it.
+// Edges of a numbering with locality stay as they are.  Sorted by the distance
+// between their cells inside chunks of 1024, so that a warp's lanes step through
+// both cells together, they touch a tenth fewer lines, which gave 2% at 720k
+// FP32 and 3 to 5% in FP64, but made a program's first iterations 6% slower.
+constexpr int kCoordSteps = 65536;
 
 // the lists with the edges' places (entry = index << 1 | negate)
 __global__ void k_order_lists(size_t n, int na, const int *__restrict__ ell,
@@ -1869,18 +1822,6 @@ __global__ void k_order_lists(size_t n, int na, const int *__restrict__ ell,
     out[i] = (k >> 1) < na ? pos[k >> 1] << 1 | (k & 1) : k;
   }
 }
-
-// A numbering without locality makes every gather of the pass a sector of its
-// own: 192 bytes an edge besides its 32, and each cell and node fetched for
-// every edge it is on.  The nodes' coordinates then order all edges: strips of
-// equal numbers of edges along the first coordinate, each by the second, so
-// that a CTA's edges share cells and nodes, which L1 keeps.  (Coordinates are a
-// guess -- res_calc's first dataset, two reals per node -- and the order is
-// dropped when a sample of it is no better.)  A counting sort: the strips by a
-// histogram of the first coordinate in 65,536 steps, then one bin per strip
-// and step of the second.  Edges of one bin lie in any order; the sums do not
-// depend on it.
-constexpr int kCoordSteps = 65536;
 
 // distinct cells on a chunk's edges
 __global__ void __launch_bounds__(kOrderChunk)
@@ -1999,6 +1940,7 @@ static bool coord_order(int na, int nnode, const int2 *edge, const int2 *cell, c
 }
 
 const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq, op_dat x) {
+  if (!sp->scattered) return nullptr;
   for (auto &o : sp->orders)
     if (o->mx == mx && o->mq == mq) return o->d_rows ? o.get() : nullptr;
   cudaStream_t s = rt().stream;
@@ -2012,59 +1954,40 @@ const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq, op_dat
   std::unique_ptr<SlotPlan::Order> o(new SlotPlan::Order());
   o->mx = mx;
   o->mq = mq;
-  o->d_rows = nullptr;
-  o->d_ell = nullptr;
-  // what it would give, from at most 128 chunks: a twentieth fewer lines at
-  // least, or the loop's own maps do.  Three of a lane's four gathers on a line
-  // of its own: no locality (a mesh numbered along its rows has less than one)
-  unsigned long long *cost = nullptr, h[2] = {0, 0};
-  int *pos = nullptr;
-  if (pool_malloc_async((void **)&cost, sizeof h, s) != cudaSuccess) {
+  o->d_rows = (int4 *)dev_alloc(sizeof(int4) * (size_t)na);
+  o->d_ell = (int *)dev_alloc(sizeof(int) * nlist);
+  // edges' places | distinct cells of a sample of the new order, of the old
+  int *mem = nullptr;
+  const size_t words = ((size_t)na + 1) / 2 * 2;
+  bool good = o->d_rows && o->d_ell &&
+              pool_malloc_async((void **)&mem, sizeof(int) * words + 16, s) == cudaSuccess;
+  unsigned long long *count = (unsigned long long *)(mem + words), h[2] = {0, 0};
+  if (good) {
+    const int nnode = x->set->size;
+    good = strcmp(x->type, "double") == 0
+               ? coord_order(na, nnode, edge, cell, (const double *)x->data_d, o->d_rows, mem, s)
+               : coord_order(na, nnode, edge, cell, (const float *)x->data_d, o->d_rows, mem, s);
+  }
+  if (good) {
+    // a quarter fewer distinct cells, or the coordinates were none
+    const int step = (nchunk + 127) / 128, nsample = (nchunk + step - 1) / step;
+    OP2B_CUDA(cudaMemsetAsync(count, 0, sizeof h, s));
+    k_chunk_cells<<<nsample, kOrderChunk, 0, s>>>(step, na, nullptr, o->d_rows, count);
+    k_chunk_cells<<<nsample, kOrderChunk, 0, s>>>(step, na, cell, nullptr, count + 1);
+    OP2B_CUDA(cudaMemcpyAsync(h, count, sizeof h, cudaMemcpyDeviceToHost, s));
+    OP2B_CUDA(cudaStreamSynchronize(s));
+    good = (double)h[0] < 0.75 * (double)h[1];
+  }
+  if (good) {
+    k_order_lists<<<rt().num_sms * 8, 256, 0, s>>>(nlist, na, sp->d_ell, mem, o->d_ell);
+  } else {
     cudaGetLastError();
-    return nullptr;
+    dev_free(o->d_rows);
+    dev_free(o->d_ell);
+    o->d_rows = nullptr;
+    o->d_ell = nullptr;
   }
-  const int step = (nchunk + 127) / 128, nsample = (nchunk + step - 1) / step;
-  OP2B_CUDA(cudaMemsetAsync(cost, 0, sizeof h, s));
-  k_flux_order<<<nsample, kOrderChunk, 0, s>>>(step, na, edge, cell, nullptr, nullptr, cost);
-  OP2B_CUDA(cudaMemcpyAsync(h, cost, sizeof h, cudaMemcpyDeviceToHost, s));
-  OP2B_CUDA(cudaStreamSynchronize(s));
-  const long long sampled = std::min((long long)nsample * kOrderChunk, (long long)na);
-  const bool scattered = (long long)h[0] > 3 * sampled;
-  const bool lines = !scattered && (double)h[1] <= 0.95 * (double)h[0];
-  if ((lines || scattered) &&
-      pool_malloc_async((void **)&pos, sizeof(int) * (size_t)na, s) == cudaSuccess) {
-    o->d_rows = (int4 *)dev_alloc(sizeof(int4) * (size_t)na);
-    o->d_ell = (int *)dev_alloc(sizeof(int) * nlist);
-    bool good = o->d_rows && o->d_ell;
-    if (good && lines) {
-      k_flux_order<<<nchunk, kOrderChunk, 0, s>>>(1, na, edge, cell, o->d_rows, pos, nullptr);
-    } else if (good) {
-      const int nnode = x->set->size;
-      good = strcmp(x->type, "double") == 0
-                 ? coord_order(na, nnode, edge, cell, (const double *)x->data_d, o->d_rows, pos, s)
-                 : coord_order(na, nnode, edge, cell, (const float *)x->data_d, o->d_rows, pos, s);
-      // a sample of the new order has a quarter fewer distinct cells than the
-      // old, or the coordinates were none
-      OP2B_CUDA(cudaMemsetAsync(cost, 0, sizeof h, s));
-      if (good) {
-        k_chunk_cells<<<nsample, kOrderChunk, 0, s>>>(step, na, nullptr, o->d_rows, cost);
-        k_chunk_cells<<<nsample, kOrderChunk, 0, s>>>(step, na, cell, nullptr, cost + 1);
-      }
-      OP2B_CUDA(cudaMemcpyAsync(h, cost, sizeof h, cudaMemcpyDeviceToHost, s));
-      OP2B_CUDA(cudaStreamSynchronize(s));
-      good = good && (double)h[0] < 0.75 * (double)h[1];
-    }
-    if (good) {
-      k_order_lists<<<rt().num_sms * 8, 256, 0, s>>>(nlist, na, sp->d_ell, pos, o->d_ell);
-    } else {
-      dev_free(o->d_rows);
-      dev_free(o->d_ell);
-      o->d_rows = nullptr;
-    }
-    OP2B_CUDA(cudaFreeAsync(pos, s));
-  }
-  OP2B_CUDA(cudaFreeAsync(cost, s));
-  cudaGetLastError();
+  if (mem) OP2B_CUDA(cudaFreeAsync(mem, s));
   sp->orders.push_back(std::move(o));
   return sp->orders.back()->d_rows ? sp->orders.back().get() : nullptr;
 }

@@ -99,6 +99,7 @@ struct SlotPlan {
     int *d_ell;             // the lists, with the places of the edges' values
   };
   std::vector<std::unique_ptr<Order>> orders;
+  bool scattered = false;  // a's elements, in order, reach targets without locality
   struct Coloured {  // get_coloured_lists
     const DevPlan *p, *pb;
     const Order *o;

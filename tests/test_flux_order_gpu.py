@@ -1,8 +1,8 @@
 """The flux pass's own order of the edges (knob flux_order) against the loop's:
 every field bit for bit, over sizes around a chunk of 1024 edges, numberings
 with and without locality, both precisions, GATHER and COLOURED, the residual
-alone and the fused chain; and the knob changed between two loops whose flux
-pass has run ahead."""
+alone and the fused chain; node datasets that are no coordinates; and the knob
+changed between two loops whose flux pass has run ahead."""
 import numpy as np
 import pytest
 
@@ -40,7 +40,7 @@ def solve(mesh, dt, strategy, order, flip=False):
 
 @pytest.mark.parametrize("dt", [np.float32, np.float64])
 @pytest.mark.parametrize("I,J,scramble", [(2, 4, False), (17, 10, False), (19, 9, False), (40, 60, False),
-                                          (60, 90, True), (131, 77, False)])
+                                          (17, 10, True), (60, 90, True), (131, 77, True)])
 def test_same_fields(dt, I, J, scramble):
     mesh = M.naca0012(I, J, scramble=scramble)
     for strategy in (api.STRATEGY_GATHER, api.STRATEGY_COLOURED):
@@ -50,3 +50,22 @@ def test_same_fields(dt, I, J, scramble):
         for k in a:
             assert a[k].tobytes() == b[k].tobytes() == c[k].tobytes(), (strategy, k)
         assert ra == rb == rc
+
+
+@pytest.mark.parametrize("what", ["nan", "inf", "same", "noise"])
+def test_node_data_that_are_no_coordinates(what):
+    mesh = M.naca0012(50, 70, scramble=True)
+    x = mesh.x32.copy()
+    if what == "nan":
+        x[::3] = np.nan
+    elif what == "inf":
+        x[::5, 0], x[::7, 1] = np.inf, -np.inf
+    elif what == "same":
+        x[:] = 1.5
+    else:
+        x[:] = np.random.default_rng(1).uniform(-1, 1, x.shape)
+    mesh.x32 = x
+    a, _ = solve(mesh, np.float32, api.STRATEGY_GATHER, 0)
+    b, _ = solve(mesh, np.float32, api.STRATEGY_GATHER, 1)
+    for k in a:
+        assert a[k].tobytes() == b[k].tobytes(), k
