@@ -1560,7 +1560,7 @@ static void update_t(char const *name, op_set set, const op_arg *args) {
     else launch(k_update<T, 4>);
     if (seq) {
       T init = *(const T *)args[4].data;
-      seq_sum<T>(seqbuf, 4LL * n, init, result, perm_old2new_dev(set), 4);
+      flag_seq = seq_sum<T>(seqbuf, 4LL * n, init, result, perm_old2new_dev(set), 4, slot);
     }
   }
   red_finish({GblRequest{args[4].data, slot, OP_INC, sizeof(T) == 8 ? GBL_F64 : GBL_F32, seq,
@@ -2174,7 +2174,7 @@ static bool persist_chain(const std::string &name, SlotPlan *sp, const op_arg *r
   }
   if (seq) {
     T init = *(const T *)ua[4].data;
-    seq_sum<T>(seqbuf, 4LL * ncell, init, result, perm_old2new_dev(ra[6].dat->set), 4);
+    seq_sum<T>(seqbuf, 4LL * ncell, init, result, perm_old2new_dev(ra[6].dat->set), 4, rslot_id);
   }
   return true;
 }
@@ -2661,7 +2661,7 @@ static bool tiled_chain(const std::string &name, SlotPlan *sp, const op_arg *ra,
   if (flip_adt) flip(adt, capturing);
   if (seq) {
     T init = *(const T *)ua[4].data;
-    seq_sum<T>(seqbuf, 4LL * ncell, init, result, perm_old2new_dev(ra[6].dat->set), 4);
+    seq_sum<T>(seqbuf, 4LL * ncell, init, result, perm_old2new_dev(ra[6].dat->set), 4, rslot_id);
   }
   return true;
 }
@@ -2848,7 +2848,8 @@ static bool res_chain_t(char const *loop_name, op_set rset, const op_arg *ra, op
 #undef OP2B_FOLD_COL
       if (seq) {
         T init = *(const T *)ua[4].data;
-        seq_sum<T>(seqbuf, 4LL * ncell, init, result, perm_old2new_dev(ra[6].dat->set), 4);
+        tail_seq = seq_sum<T>(seqbuf, 4LL * ncell, init, result,
+                              perm_old2new_dev(ra[6].dat->set), 4, rslot_id);
       }
     }
     }

@@ -279,7 +279,9 @@ void *red_seq_buffer(size_t bytes) {
 }
 
 template <class T>
-void seq_sum(const T *v, long long n, T init, T *out, const int *order, int w) {
+unsigned seq_sum(const T *v, long long n, T init, T *out, const int *order, int w, int slot) {
+  unsigned *flag;
+  const unsigned seq = red_flag(slot, &flag);
   const int ntile = (int)std::max(1LL, (n + kSeqTile - 1) / kSeqTile);
   char *tab = (char *)v + seq_table_offset(sizeof(T) * (size_t)n);
   double *tsum = (double *)tab;
@@ -289,10 +291,12 @@ void seq_sum(const T *v, long long n, T init, T *out, const int *order, int w) {
   cudaStream_t s = rt().stream;
   launch_pdl(k_seq_tile_sums<T>, ntile, kSeqThreads, 0, s, a, tsum);
   launch_pdl(k_seq_fold<T>, ntile, kSeqThreads, 0, s, a, init, ntile, (const double *)tsum, tiles,
-             runs, binade, red_ticket() + 1, out);
+             runs, binade, red_ticket() + 1, out, flag, seq);
+  return seq;
 }
-template void seq_sum<float>(const float *, long long, float, float *, const int *, int);
-template void seq_sum<double>(const double *, long long, double, double *, const int *, int);
+template unsigned seq_sum<float>(const float *, long long, float, float *, const int *, int, int);
+template unsigned seq_sum<double>(const double *, long long, double, double *, const int *, int,
+                                  int);
 
 int red_grid(long long n, int threads) {
   long long want = (n + threads - 1) / threads;

@@ -345,7 +345,8 @@ static void jac_update_t(char const *name, op_set set, const op_arg *args,
       flag_seq = red_tail_leave(GBL_F32, grid, slot_sum, slot_max, 8,
                                 kernel_nparams(k_jac_update<V>));
     if (seq)
-      seq_sum<float>(seqbuf, n, *(const float *)args[3].data, r_sum, perm_old2new_dev(set), 1);
+      flag_seq = seq_sum<float>(seqbuf, n, *(const float *)args[3].data, r_sum,
+                                perm_old2new_dev(set), 1, slot_sum);
   }
   std::vector<GblRequest> rq{GblRequest{args[3].data, slot_sum, OP_INC, GBL_F32, seq, flag_seq, slot_sum},
                              GblRequest{args[4].data, slot_max, OP_MAX, GBL_F32, false, flag_seq,
@@ -603,7 +604,8 @@ bool run_jac_step(char const *uname, op_set uset, const op_arg *ua, char const *
                (const float *)r->data_d, (const float *)du->data_d, (const float *)u->data_d,
                alpha, beta, u_out, du_out, seqbuf, ss, sm, red_ticket());
     if (seq)
-      seq_sum<float>(seqbuf, n, *(const float *)ua[3].data, r_sum, perm_old2new_dev(uset), 1);
+      seq_sum<float>(seqbuf, n, *(const float *)ua[3].data, r_sum, perm_old2new_dev(uset), 1,
+                     slot_sum);
   }
   if (error_pending()) return true;
   flip(u, capturing);

@@ -53,9 +53,10 @@ int red_new_slot();
 unsigned red_flag(int slot, unsigned **flag);
 void *red_seq_buffer(size_t bytes);  // scratch for SEQ-mode contributions
 // *out = init + v[0] + v[1] + ... + v[n-1], added in that order (value j of a
-// renumbered set: see SeqVals); v is red_seq_buffer's
+// renumbered set: see SeqVals); v is red_seq_buffer's, out the slot's place.
+// Returns the number the slot's flag will have (red_flag)
 template <class T>
-void seq_sum(const T *v, long long n, T init, T *out, const int *order, int w);
+unsigned seq_sum(const T *v, long long n, T init, T *out, const int *order, int w, int slot);
 // The kernel just launched wrote its n block partials (in red_partials) of a
 // sum, and of a maximum when slot_max >= 0, and left them unfolded: the next
 // kernel that takes the tail folds them, or red_tail_flush does.  Returns the
