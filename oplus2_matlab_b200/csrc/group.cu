@@ -21,12 +21,12 @@
 // solve.  The first update's rms is not computed: the reference app zeroes it
 // before the second update (airfoil/airfoil_op.cpp:283-290).
 //
-// The second update's rms: every cell tile of a solve writes one partial
-// (its threads' sums, folded in a fixed tree); the last CTA of the solve to
-// finish (a per-solve ticket) folds the solve's partials in tile order,
-// stores sqrt(sum / ncell) in the solve's history, advances its iteration
-// count and applies the stopping test.  Tiles are fixed by the solve's own
-// cell count (kCellTile), so the rms does not depend on the other solves.
+// The second update's rms: every 256 consecutive cells of a solve make one
+// partial (folded in a fixed tree); the last CTA of the solve to finish (a
+// per-solve ticket) folds the solve's partials in order, stores
+// sqrt(sum / ncell) in the solve's history, advances its iteration count and
+// applies the stopping test.  Whatever run of cells a CTA takes, the partials
+// are the same, so the rms does not depend on the other solves.
 // A stopped solve's CTAs return at once; the host drops it from the tile
 // tables at the next op2b_group_run after a poll.
 
@@ -48,8 +48,8 @@ namespace op2b {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kCellsPerThread = 4;
-constexpr int kCellTile = kThreads * kCellsPerThread;  // fixes the rms fold order
+constexpr int kCellTile = 4 * kThreads;  // cells of a save_soln + adt_calc CTA
+constexpr int kMaxCellRun = 4;           // times kThreads cells: a fold CTA's longest run (a warp each)
 constexpr int kMaxWidth = 8;                           // longest contribution list
 
 template <class T>
@@ -57,7 +57,7 @@ struct SolveDev {  // device view of one solve; written by the host only
   const T *x;
   T *q, *qold, *adt, *vals, *partials, *hist;
   const int *pedge, *pecell, *pbedge, *pbecell, *bound, *pcell, *ell;
-  int ncell, nedge, nbedge, W, ntiles, pad;
+  int ncell, nedge, nbedge, W;
   T qinf[4];
   // the tiled chain: second buffers of q and adt, and the tile lists
   T *q2, *adt2;
@@ -86,30 +86,30 @@ __device__ __forceinline__ AirConsts<T> with_qinf(AirConsts<T> K, const SolveDev
   return K;
 }
 
-// The end of an iteration's second update: this CTA's rms partial (its
-// threads' sums, block tree) into the solve's slot for the tile; the
-// solve's last CTA folds the ntiles partials in tile order, records
-// rms = sqrt(sum / ncell) (airfoil/airfoil_op.cpp:291) and applies the
-// stopping test (iteration cap, or rms below tol x the first iteration's)
+// The end of an iteration's second update, after this CTA's partials are
+// written and its threads have met: the last of the solve's ctas CTAs folds
+// the solve's n partials in their order, records rms = sqrt(sum / ncell)
+// (airfoil/airfoil_op.cpp:291) and applies the stopping test (iteration cap,
+// or rms below tol x the first iteration's).  Thread 0's fence covers every
+// writer's partial; one of each writer's as well took another 3 us of an
+// iteration of 162 (a CTA lives for some 10 us)
 template <class T>
-__device__ __forceinline__ void end_of_iteration(const SolveDev<T> *d, SolveState *st,
-                                                 const Tile &t, T rms, int ntiles) {
+__device__ __forceinline__ void end_of_iteration(const SolveDev<T> *d, SolveState *st, int solve,
+                                                 int ctas, int n) {
   __shared__ T ws[32];
   __shared__ bool last;
-  const T b = block_fold(rms, T(0), OpSum(), ws);
-  if (threadIdx.x == 0) {  // the writer fences its partial, then takes a ticket
-    d->partials[t.local] = b;
+  if (threadIdx.x == 0) {
     __threadfence();
-    last = atomicAdd(&st[t.solve].ticket, 1u) == (unsigned)(ntiles - 1);
+    last = atomicAdd(&st[solve].ticket, 1u) == (unsigned)(ctas - 1);
   }
   __syncthreads();
   if (!last) return;
   __threadfence();
   T sum = T(0);
-  for (int p = threadIdx.x; p < ntiles; p += blockDim.x) sum += __ldcg(d->partials + p);
+  for (int p = threadIdx.x; p < n; p += blockDim.x) sum += __ldcg(d->partials + p);
   sum = block_fold(sum, T(0), OpSum(), ws);
   if (threadIdx.x == 0) {
-    SolveState &s = st[t.solve];
+    SolveState &s = st[solve];
     const T r = sqrt(sum / (T)d->ncell);
     const int it = s.iter;
     d->hist[it] = r;
@@ -217,11 +217,19 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 8 : 4)
 // iteration's save_soln and adt_calc on the new q (qold = q, then adt), so
 // that iteration starts at its res_calc; update reads qold at the cell
 // before the copy overwrites it, hence the coherent load
+//
+// Bound: DRAM for groups past the L2 (12 solves, 1.96M cells FP32: 41 and 52
+// us against 37 and 42 for the bytes), the latency of one cell's chain of
+// loads for small ones, whose CTAs take 256 cells each (cell_run).  The plain
+// path's k_fold_cells form (every load of the next cell ahead, 2 CTAs per SM)
+// was slower here on large groups, 171 against 162 us an iteration: past the
+// L2 more warps in flight beat more loads per warp.
 template <class T, int MODE>
 __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? (MODE == 1 ? 4 : 3) : 2)
     k_grp_fold(const Tile *__restrict__ tiles, const SolveDev<T> *__restrict__ sd,
                SolveState *st, AirConsts<T> K) {
   constexpr bool FIRST = MODE == 0, ADT = MODE != 1, SAVE = MODE == 2;
+  __shared__ T part[FIRST ? 1 : kMaxCellRun][FIRST ? 1 : kThreads];
   const Tile t = tiles[blockIdx.x];
   const SolveDev<T> *d = sd + t.solve;
   const int W = d->W;
@@ -241,7 +249,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? (MODE == 1 ? 4 : 3)
   if (!live) return;
   const T *x = d->x, *qold = d->qold, *vals = d->vals;
   T *q = d->q, *adt = d->adt;
-  T rms = T(0);
+  int step = 0;
 #pragma unroll 1
   for (int i = threadIdx.x; i < t.count; i += kThreads) {
     const int c = t.start + i;
@@ -250,8 +258,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? (MODE == 1 ? 4 : 3)
     else ld4(qold + 4 * (size_t)c, qo);
     const T ad = adt[c];
 #pragma unroll
-    for (int m = 0; m < 4; m++)
-      if (k[m] >= 0) ld4(vals + 4 * (size_t)(k[m] >> 1), f[m]);
+    for (int m = 0; m < 4; m++) ld4(vals + 4 * (size_t)(k[m] >> 1), f[m]);
     if (ADT) {
       ld2(x + 2 * (size_t)nd.x, xs[0]);
       ld2(x + 2 * (size_t)nd.y, xs[1]);
@@ -264,15 +271,16 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? (MODE == 1 ? 4 : 3)
       if (ADT) nd = ld_stream(pcell + c + kThreads);
     }
 #pragma unroll
-    for (int m = 0; m < 4; m++) add_listed(r, kc[m], f[m]);
+    for (int m = 0; m < 4; m++) add_signed(r, kc[m], f[m]);
     for (int m = 4; m < W; m++) {  // lists longer than 4
       const int kk = __ldg(ell + (size_t)c * W + m);
       T g[4];
       ld4(vals + 4 * (size_t)(kk >> 1), g);
-      add_listed(r, kk, g);
+      add_signed(r, kk, g);
     }
     const T adti = rcp(ad);
-    T qn[4];
+    T qn[4], rms = T(0);
+#pragma unroll
     for (int m = 0; m < 4; m++) {
       const T del = adti * r[m];
       qn[m] = qo[m] - del;
@@ -281,9 +289,22 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? (MODE == 1 ? 4 : 3)
     st4(q + 4 * (size_t)c, qn);
     if (SAVE) st4(d->qold + 4 * (size_t)c, qn);  // airfoil/save_soln.h:1-3
     if (ADT) adt[c] = adt_calc(xs[0], xs[1], xs[2], xs[3], qn, K);
+    if (!FIRST) part[step++][threadIdx.x] = rms;
   }
   if (FIRST) return;
-  end_of_iteration(d, st, t, rms, d->ntiles);
+  const int steps = (t.count + kThreads - 1) / kThreads;
+  if (step < steps) part[step][threadIdx.x] = T(0);
+  __syncthreads();
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (w < steps) {
+    T s = T(0);
+#pragma unroll
+    for (int j = 0; j < kThreads; j += 32) s += part[w][j + lane];
+    s = warp_fold(s, OpSum());
+    if (lane == 0) d->partials[t.start / kThreads + w] = s;
+  }
+  __syncthreads();
+  end_of_iteration(d, st, t.solve, t.local, (d->ncell + kThreads - 1) / kThreads);
 }
 
 // The tiled chain over one tile of one solve's cells per CTA
@@ -333,7 +354,10 @@ __global__ void __launch_bounds__(1024, 1)
       t.start, t.start + t.count, d->tell, d->W, reinterpret_cast<const int4 *>(d->pcell), x,
       d->qold, ain, qout, nullptr, d->qold, aout, nullptr, K, fv);
   if (FIRST) return;
-  end_of_iteration(d, st, t, rms, d->tntile);
+  __shared__ T ws[32];
+  const T b = block_fold(rms, T(0), OpSum(), ws);
+  if (threadIdx.x == 0) d->partials[t.local] = b;
+  end_of_iteration(d, st, t.solve, d->tntile, d->tntile);
 }
 
 // ------------------------------------------------ contribution lists ------
@@ -528,7 +552,16 @@ struct Group : GroupBase {
   int etile = 2048;
   bool etile_auto = true;  // until it is set or tuned
   bool changed = true;
-  cudaGraphExec_t exec = nullptr;
+  // one iteration, and kUnroll of them in one graph: the next iteration's first
+  // launch then overlaps the end of the one before, which a graph's boundary
+  // does not let it (3 solves, 42k cells: 15.0 -> 13.6 us an iteration, FP64
+  // 19.7 -> 17.8; 12 solves 162.8 -> 161.6).  Made by the first run that takes
+  // them, which a short run right after the tiles were made does not: it
+  // issues its launches one by one, for less than a graph costs to make (first
+  // 30 iterations of the 3 solves: 2.77 -> 2.58 ms)
+  static constexpr int kUnroll = 8;
+  cudaGraphExec_t exec = nullptr, exec_many = nullptr;
+  bool fresh = true;  // no iteration since the tiles were made
   cudaEvent_t mirror_ev = nullptr;
   bool mirror_pending = false;
   long long mirror_epoch = 0;  // state mirrors issued (run) so far
@@ -552,7 +585,7 @@ struct Group : GroupBase {
     if (cs) cudaStreamSynchronize(cs);
     if (us) cudaStreamSynchronize(us);
     for (auto &s : solves) release(s);
-    if (exec) cudaGraphExecDestroy(exec);
+    drop_graphs();
     cudaFree(d_sd);
     cudaFree(d_st);
     cudaFree(d_ct);
@@ -587,14 +620,14 @@ struct Group : GroupBase {
   }
 
   static size_t layout(int nn, int nc, int ne, int nb, int max_iter, size_t off[16]) {
-    const int ntiles = (nc + kCellTile - 1) / kCellTile;
+    const int nparts = (nc + kThreads - 1) / kThreads;
     const size_t sz[16] = {sizeof(T) * 2 * (size_t)nn,                 // x
                            sizeof(T) * 4 * (size_t)nc,                 // q
                            sizeof(T) * 4 * (size_t)nc,                 // qold
                            sizeof(T) * (size_t)nc,                     // adt
                            0,                                          // (res: none)
                            sizeof(T) * 4 * ((size_t)ne + nb + 1),      // vals
-                           sizeof(T) * (size_t)std::max(ntiles, 1),    // partials
+                           sizeof(T) * (size_t)std::max(nparts, 1),    // partials
                            sizeof(T) * (size_t)std::max(max_iter, 1),  // hist
                            sizeof(int) * 2 * (size_t)ne,               // pedge
                            sizeof(int) * 2 * (size_t)ne,               // pecell
@@ -721,7 +754,6 @@ struct Group : GroupBase {
     d.bound = (const int *)(b + off[12]); d.pcell = (const int *)(b + off[13]);
     int *cnt = (int *)(b + off[14]);
     d.ncell = s.ncell; d.nedge = s.nedge; d.nbedge = s.nbedge;
-    d.ntiles = (s.ncell + kCellTile - 1) / kCellTile;
     T c4[4];
     flow_state<T>(mach, alpha, d.qinf, c4);
     const T *xh = (const T *)(sizeof(T) == 8 ? (const void *)m->x64 : (const void *)m->x32);
@@ -749,6 +781,7 @@ struct Group : GroupBase {
            kMaxWidth);
       return -1;
     }
+    W = std::max(W, 4);  // lists of at least four, so four are always there to load
     d.W = W;
     if (pool_malloc_async((void **)&s.ell, sizeof(int) * W * (size_t)s.ncell, us) != cudaSuccess) {
       cudaGetLastError();
@@ -828,6 +861,7 @@ struct Group : GroupBase {
   // up to block_bytes of values (a larger solve makes a block of its own).
   struct Block {
     int ct0, nct, et0, net, tt0, ntt;
+    int ids;  // solves up to its last
   };
   std::vector<Block> blocks;
   // default one block: measured on 64 solves (12M cells), blocks of 24, 48
@@ -836,8 +870,25 @@ struct Group : GroupBase {
   // DRAM round trip of the values); the autotuner tries them all
   size_t block_bytes = ~(size_t)0;
 
+  // Cells of a fold CTA's threads (times kThreads: its run): as few as let the
+  // CTAs of all these solves be resident together (3 per SM in FP32, 2 in
+  // FP64), or the longest run, in several waves.  Iteration of 3 solves, 42k
+  // cells: FP32 20.9 -> 16.8 us at 256 cells against 1024, FP64 25.7 -> 20.9;
+  // 12 solves, 1.96M cells: 164 us at 1024 cells, 166 at 2048, 174 at 512
+  int cell_run(const std::vector<int> &ids) const {
+    const long long slots = (long long)rt().num_sms * (sizeof(T) == 4 ? 3 : 2);
+    int r = 1;
+    for (; r < kMaxCellRun; r *= 2) {
+      long long ctas = 0;
+      for (int id : ids) ctas += (solves[id].ncell + r * kThreads - 1LL) / (r * kThreads);
+      if (ctas <= slots) break;
+    }
+    return r;
+  }
+
   void rebuild() {
     std::vector<Tile> ct, et, pt, tt;
+    std::vector<int> ids;  // of the blocks' solves
     blocks.clear();
     nactive = 0;
     graph_cells = stopped_cells = 0;
@@ -872,12 +923,11 @@ struct Group : GroupBase {
       const int nv = s.nedge + s.nbedge;
       const size_t vbytes = sizeof(T) * 4 * (size_t)nv;
       if (blocks.empty() || (in_block > 0 && in_block + vbytes > block_bytes)) {
-        blocks.push_back(Block{(int)ct.size(), 0, (int)et.size(), 0, (int)tt.size(), 0});
+        blocks.push_back(Block{0, 0, (int)et.size(), 0, (int)tt.size(), 0, 0});
         in_block = 0;
       }
       in_block += vbytes;
-      for (int a = 0, l = 0; a < s.ncell; a += kCellTile, l++)
-        ct.push_back(Tile{id, a, std::min(kCellTile, s.ncell - a), l});
+      ids.push_back(id);
       for (int a = 0, l = 0; a < nv; a += etile, l++)
         et.push_back(Tile{id, a, std::min(etile, nv - a), l});
       if (tiled) {
@@ -885,9 +935,21 @@ struct Group : GroupBase {
           tt.push_back(Tile{id, a, std::min(s.tl.ct, s.ncell - a), l});
         tsmem = std::max(tsmem, (size_t)s.tl.maxcnt * 4 * sizeof(T));
       }
-      blocks.back().nct = (int)ct.size() - blocks.back().ct0;
+      blocks.back().ids = (int)ids.size();
       blocks.back().net = (int)et.size() - blocks.back().et0;
       blocks.back().ntt = (int)tt.size() - blocks.back().tt0;
+    }
+    for (size_t i = 0, first = 0; i < blocks.size(); i++) {
+      Block &b = blocks[i];
+      const std::vector<int> mine(ids.begin() + first, ids.begin() + b.ids);
+      first = b.ids;
+      b.ct0 = (int)ct.size();
+      const int run = kThreads * cell_run(mine);
+      for (int id : mine) {
+        const int nc = solves[id].ncell, n = (nc + run - 1) / run;
+        for (int a = 0; a < nc; a += run) ct.push_back(Tile{id, a, std::min(run, nc - a), n});
+      }
+      b.nct = (int)ct.size() - b.ct0;
     }
     upload_tiles(d_ct, ct_cap, ct);
     upload_tiles(d_et, et_cap, et);
@@ -904,14 +966,10 @@ struct Group : GroupBase {
         OP2B_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem));
       tsmem_set = tsmem;
     }
-    if (exec) {
-      cudaGraphExecDestroy(exec);
-      exec = nullptr;
-    }
-    if (nactive == 0) return;
-    cudaGraph_t graph = nullptr;
+    drop_graphs();
+    fresh = true;
     const int K = std::max(1, std::min(nstreams, (int)blocks.size()));
-    while ((int)side.size() < K - 1) {  // created outside the capture
+    while ((int)side.size() < K - 1) {  // created outside a capture
       cudaStream_t x;
       OP2B_CUDA(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
       side.push_back(x);
@@ -921,24 +979,65 @@ struct Group : GroupBase {
       OP2B_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
       side_ev.push_back(e);
     }
-    OP2B_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
+    changed = false;
+  }
+
+  void drop_graphs() {
+    for (cudaGraphExec_t *e : {&exec, &exec_many}) {
+      if (*e) cudaGraphExecDestroy(*e);
+      *e = nullptr;
+    }
+  }
+
+  // reps iterations of the blocks as they are, on cs and the side streams
+  void enqueue(int reps) {
+    const int K = std::max(1, std::min(nstreams, (int)blocks.size()));
     if (K > 1) {
       OP2B_CUDA(cudaEventRecord(side_ev[0], cs));
       for (int k = 1; k < K; k++) OP2B_CUDA(cudaStreamWaitEvent(side[k - 1], side_ev[0], 0));
     }
-    for (size_t i = 0; i < blocks.size(); i++)
-      iteration(blocks[i], i % K == 0 ? cs : side[i % K - 1]);
+    for (int r = 0; r < reps; r++)
+      for (size_t i = 0; i < blocks.size(); i++)
+        iteration(blocks[i], i % K == 0 ? cs : side[i % K - 1]);
     if (K > 1)
       for (int k = 1; k < K; k++) {
         OP2B_CUDA(cudaEventRecord(side_ev[k], side[k - 1]));
         OP2B_CUDA(cudaStreamWaitEvent(cs, side_ev[k], 0));
       }
+  }
+
+  cudaGraphExec_t capture(int reps) {
+    cudaGraphExec_t e = nullptr;
+    cudaGraph_t graph = nullptr;
+    OP2B_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
+    enqueue(reps);
     OP2B_CUDA(cudaStreamEndCapture(cs, &graph));
     if (graph) {
-      OP2B_CUDA(cudaGraphInstantiate(&exec, graph, 0));
+      OP2B_CUDA(cudaGraphInstantiate(&e, graph, 0));
       cudaGraphDestroy(graph);
     }
-    changed = false;
+    return e;
+  }
+
+  // the graphs that n iterations take
+  void make_graphs(int n) {
+    if (nactive == 0 || n <= 0) return;
+    cudaGraphExec_t &e = n >= kUnroll ? exec_many : exec;
+    if (!e) e = capture(n >= kUnroll ? kUnroll : 1);
+  }
+
+  // n iterations of the active solves
+  void iterate(int n) {
+    if (nactive == 0 || n <= 0) return;
+    if (!exec && !exec_many && fresh && n < 8 * kUnroll) {
+      enqueue(n);
+    } else if (make_graphs(n); n >= kUnroll) {
+      for (; n >= kUnroll && exec_many; n -= kUnroll) OP2B_CUDA(cudaGraphLaunch(exec_many, cs));
+      enqueue(n);  // the rest are issued while those run
+    } else {
+      for (; n > 0 && exec; n--) OP2B_CUDA(cudaGraphLaunch(exec, cs));
+    }
+    fresh = false;
   }
 
   void iteration(const Block &b, cudaStream_t cs) {
@@ -1011,9 +1110,10 @@ struct Group : GroupBase {
     if (error_pending()) return -1;
     if (changed) rebuild();
     if (error_pending()) return -1;
-    if (exec && niter > 0) prime();
-    if (exec)
-      for (int i = 0; i < niter; i++) OP2B_CUDA(cudaGraphLaunch(exec, cs));
+    if (nactive > 0 && niter > 0) {
+      prime();
+      iterate(niter);
+    }
     if ((int)solves.size() > 0 && cap > 0) {
       OP2B_CUDA(cudaMemcpyAsync(h_st, d_st, sizeof(SolveState) * solves.size(),
                                 cudaMemcpyDeviceToHost, cs));
@@ -1226,9 +1326,10 @@ struct Group : GroupBase {
     OP2B_CUDA(cudaEventCreate(&e1));
     auto trial = [&]() {
       rebuild();
-      OP2B_CUDA(cudaGraphLaunch(exec, cs));  // warm
+      make_graphs(iters);
+      iterate(iters >= kUnroll ? kUnroll : 1);  // warm
       OP2B_CUDA(cudaEventRecord(e0, cs));
-      for (int i = 0; i < iters; i++) OP2B_CUDA(cudaGraphLaunch(exec, cs));
+      iterate(iters);
       OP2B_CUDA(cudaEventRecord(e1, cs));
       OP2B_CUDA(cudaEventSynchronize(e1));
       float ms = 0;
@@ -1301,18 +1402,21 @@ struct Group : GroupBase {
                                           {24u << 20, 2}, {24u << 20, 3}, {12u << 20, 4}};
     for (const auto &bb : blk) trials.push_back(Trial{-1, bb.first, bb.second});
     std::vector<cudaGraphExec_t> retired;  // destroyed after the final synchronisation
+    auto retire = [&]() {
+      for (cudaGraphExec_t *e : {&exec, &exec_many}) {
+        if (*e) retired.push_back(*e);
+        *e = nullptr;
+      }
+    };
     int ran = 0;
     auto enqueue = [&](Trial &t) {
-      if (exec) {
-        retired.push_back(exec);
-        exec = nullptr;
-      }
+      retire();
       rebuild();
+      make_graphs(iters);
       OP2B_CUDA(cudaEventCreate(&t.e0));
       OP2B_CUDA(cudaEventCreate(&t.e1));
       OP2B_CUDA(cudaEventRecord(t.e0, cs));
-      if (exec)
-        for (int i = 0; i < iters; i++) OP2B_CUDA(cudaGraphLaunch(exec, cs));
+      iterate(iters);
       OP2B_CUDA(cudaEventRecord(t.e1, cs));
       ran += iters;
     };
@@ -1357,10 +1461,7 @@ struct Group : GroupBase {
     }
     block_bytes = best_blk.first;
     nstreams = best_blk.second;
-    if (exec) {
-      retired.push_back(exec);
-      exec = nullptr;
-    }
+    retire();
     rebuild();
     OP2B_CUDA(cudaStreamSynchronize(cs));
     for (cudaGraphExec_t e : retired) cudaGraphExecDestroy(e);
