@@ -555,9 +555,8 @@ struct Group : GroupBase {
   // one iteration, and kUnroll of them in one graph: the next iteration's first
   // launch then overlaps the end of the one before, which a graph's boundary
   // does not let it (3 solves, 42k cells: 15.0 -> 13.6 us an iteration, FP64
-  // 19.7 -> 17.8; 12 solves 162.8 -> 161.6).  Made by the first run that takes
-  // them, which a short run right after the tiles were made does not: it
-  // issues its launches one by one, for less than a graph costs to make (first
+  // 19.7 -> 17.8; 12 solves 162.8 -> 161.6).  A short first run makes none: its
+  // launches are issued one by one, for less than a graph costs to make (first
   // 30 iterations of the 3 solves: 2.77 -> 2.58 ms)
   static constexpr int kUnroll = 8;
   cudaGraphExec_t exec = nullptr, exec_many = nullptr;
@@ -1026,18 +1025,28 @@ struct Group : GroupBase {
     if (!e) e = capture(n >= kUnroll ? kUnroll : 1);
   }
 
-  // n iterations of the active solves
+  // n iterations of the active solves.  A graph that is not there yet is made
+  // after the first of them have been issued one by one, while those run (the
+  // first 39 iterations after a short run, 3 solves of 17k to 339k cells: 1615
+  // -> 1390 us against making it first)
   void iterate(int n) {
     if (nactive == 0 || n <= 0) return;
-    if (!exec && !exec_many && fresh && n < 8 * kUnroll) {
-      enqueue(n);
-    } else if (make_graphs(n); n >= kUnroll) {
-      for (; n >= kUnroll && exec_many; n -= kUnroll) OP2B_CUDA(cudaGraphLaunch(exec_many, cs));
-      enqueue(n);  // the rest are issued while those run
-    } else {
-      for (; n > 0 && exec; n--) OP2B_CUDA(cudaGraphLaunch(exec, cs));
+    const int reps = n >= kUnroll ? kUnroll : 1;
+    if (!(reps == 1 ? exec : exec_many)) {
+      const int direct = std::min(n, 2 * kUnroll);
+      enqueue(direct);
+      n -= direct;
+      const bool first = fresh;
+      fresh = false;
+      if (first && n == 0) return;
+      make_graphs(reps);
     }
-    fresh = false;
+    if (reps == 1) {
+      for (; n > 0 && exec; n--) OP2B_CUDA(cudaGraphLaunch(exec, cs));
+      return;
+    }
+    for (; n >= kUnroll && exec_many; n -= kUnroll) OP2B_CUDA(cudaGraphLaunch(exec_many, cs));
+    enqueue(n);  // the rest are issued while those run
   }
 
   void iteration(const Block &b, cudaStream_t cs) {
