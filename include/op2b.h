@@ -66,8 +66,8 @@ enum { OP2B_REDUCE_TREE = 0, OP2B_REDUCE_SEQ = 1 };
  *                   of four, one x dataset) with every load of a thread's next
  *                   cell ahead of this cell's arithmetic; 0: the general pass
  *   "flux_order"    1 (default): where the numbering has no locality, the flux
- *                   pass takes the edges in the order of their nodes'
- *                   coordinates; 0: in edge order
+ *                   pass of a mesh of 16,384 or more edges takes them in the
+ *                   order of their nodes' coordinates; 0: in edge order
  *   "red_tail"      1 (default): the rms of an update is folded by the flux
  *                   pass behind it; 0: by the update's last block
  *   "coloured_fold" 1 (default): COLOURED res_calc [+ bres_calc ...] as the
