@@ -127,7 +127,7 @@ cudaError_t pool_malloc_async(void **p, size_t bytes, cudaStream_t s) {
   return mp ? cudaMallocFromPoolAsync(p, bytes, mp, s) : cudaMallocAsync(p, bytes, s);
 }
 
-void *dev_alloc(size_t bytes) {
+static cudaError_t alloc(void **out, size_t bytes) {
   void *p = nullptr;
   if (bytes == 0) bytes = 16;
   ensure_cuda();
@@ -141,10 +141,21 @@ void *dev_alloc(size_t bytes) {
   } else {
     err = cudaMalloc(&p, bytes);
   }
-  if (err != cudaSuccess) {
+  *out = err == cudaSuccess ? p : nullptr;
+  return err;
+}
+
+void *dev_alloc(size_t bytes) {
+  void *p;
+  const cudaError_t err = alloc(&p, bytes);
+  if (err != cudaSuccess)
     fail(-1, "op2b error: allocation of %zu bytes failed: %s\n", bytes, cudaGetErrorString(err));
-    return nullptr;
-  }
+  return p;
+}
+
+void *dev_try_alloc(size_t bytes) {
+  void *p;
+  if (alloc(&p, bytes) != cudaSuccess) cudaGetLastError();
   return p;
 }
 

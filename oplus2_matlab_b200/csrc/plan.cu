@@ -1657,7 +1657,7 @@ constexpr int kOrderChunk = 1024;
 // Fewer elements than these keep their order: what they read is then about what
 // one SM's L1 holds.  An iteration of a scrambled mesh in coordinate order against
 // its own: 2.5k cells 8.45 and 8.45 us, 5.2k 8.95 and 9.14, 10.5k (21k edges) 9.29
-// and 9.48, 21k 9.99 and 11.56; finding and making the order takes 130 us.
+// and 9.48, 21k 9.99 and 11.56; making the order takes 100 us.
 constexpr int kOrderLeast = 16 * kOrderChunk;
 __global__ void __launch_bounds__(kOrderChunk)
     k_target_lines(int step, int n, SlotMaps sm, int *lines) {
@@ -1819,13 +1819,25 @@ const int *get_coloured_lists(SlotPlan *sp, const SlotPlan::Order *o, const DevP
 // FP32 and 3 to 5% in FP64, but made a program's first iterations 6% slower.
 constexpr int kCoordSteps = 65536;
 
-// the lists with the edges' places (entry = index << 1 | negate)
+// the lists with the edges' places (entry = index << 1 | negate), or lists and
+// rows of the loop's order where the sample in cells (distinct cells in the new
+// order, in the old) is not a quarter smaller
 __global__ void k_order_lists(size_t n, int na, const int *__restrict__ ell,
-                              const int *__restrict__ pos, int *__restrict__ out) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
+                              const int *__restrict__ pos,
+                              const unsigned long long *__restrict__ cells,
+                              const int2 *__restrict__ edge, const int2 *__restrict__ cell,
+                              int4 *__restrict__ rows, int *__restrict__ out) {
+  const bool good = 4 * cells[0] < 3 * cells[1];
+  const size_t i0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  for (size_t i = i0; i < n; i += stride) {
     const int k = ell[i];
-    out[i] = (k >> 1) < na ? pos[k >> 1] << 1 | (k & 1) : k;
+    out[i] = good && (k >> 1) < na ? pos[k >> 1] << 1 | (k & 1) : k;
+  }
+  if (good) return;
+  for (size_t e = i0; e < (size_t)na; e += stride) {
+    const int2 m = edge[e], c = cell[e];
+    rows[e] = make_int4(m.x, m.y, c.x, c.y);
   }
 }
 
@@ -1960,14 +1972,13 @@ const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq, op_dat
   std::unique_ptr<SlotPlan::Order> o(new SlotPlan::Order());
   o->mx = mx;
   o->mq = mq;
-  o->d_rows = (int4 *)dev_alloc(sizeof(int4) * (size_t)na);
-  o->d_ell = (int *)dev_alloc(sizeof(int) * nlist);
+  o->d_rows = (int4 *)dev_try_alloc(sizeof(int4) * (size_t)na + sizeof(int) * nlist);
+  o->d_ell = (int *)(o->d_rows + (o->d_rows ? na : 0));
   // edges' places | distinct cells of a sample of the new order, of the old
   int *mem = nullptr;
   const size_t words = ((size_t)na + 1) / 2 * 2;
-  bool good = o->d_rows && o->d_ell &&
+  bool good = o->d_rows &&
               pool_malloc_async((void **)&mem, sizeof(int) * words + 16, s) == cudaSuccess;
-  unsigned long long *count = (unsigned long long *)(mem + words), h[2] = {0, 0};
   if (good) {
     const int nnode = x->set->size;
     good = strcmp(x->type, "double") == 0
@@ -1975,21 +1986,16 @@ const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq, op_dat
                : coord_order(na, nnode, edge, cell, (const float *)x->data_d, o->d_rows, mem, s);
   }
   if (good) {
-    // a quarter fewer distinct cells, or the coordinates were none
+    unsigned long long *cells = (unsigned long long *)(mem + words);
     const int step = (nchunk + 127) / 128, nsample = (nchunk + step - 1) / step;
-    OP2B_CUDA(cudaMemsetAsync(count, 0, sizeof h, s));
-    k_chunk_cells<<<nsample, kOrderChunk, 0, s>>>(step, na, nullptr, o->d_rows, count);
-    k_chunk_cells<<<nsample, kOrderChunk, 0, s>>>(step, na, cell, nullptr, count + 1);
-    OP2B_CUDA(cudaMemcpyAsync(h, count, sizeof h, cudaMemcpyDeviceToHost, s));
-    OP2B_CUDA(cudaStreamSynchronize(s));
-    good = (double)h[0] < 0.75 * (double)h[1];
-  }
-  if (good) {
-    k_order_lists<<<rt().num_sms * 8, 256, 0, s>>>(nlist, na, sp->d_ell, mem, o->d_ell);
+    OP2B_CUDA(cudaMemsetAsync(cells, 0, 2 * sizeof *cells, s));
+    k_chunk_cells<<<nsample, kOrderChunk, 0, s>>>(step, na, nullptr, o->d_rows, cells);
+    k_chunk_cells<<<nsample, kOrderChunk, 0, s>>>(step, na, cell, nullptr, cells + 1);
+    k_order_lists<<<rt().num_sms * 8, 256, 0, s>>>(nlist, na, sp->d_ell, mem, cells, edge, cell,
+                                                   o->d_rows, o->d_ell);
   } else {
     cudaGetLastError();
     dev_free(o->d_rows);
-    dev_free(o->d_ell);
     o->d_rows = nullptr;
     o->d_ell = nullptr;
   }
@@ -2011,7 +2017,6 @@ void op2b_release_plans() {
     for (auto &c : up->coloured) dev_free(c.d_ell);
     for (auto &o : up->orders) {
       dev_free(o->d_rows);
-      dev_free(o->d_ell);
     }
   }
   g_slot_plans.clear();
