@@ -1857,12 +1857,20 @@ static bool flux_pair_shape(const op_arg *ra, size_t nval) {
          (long long)ra[0].dat->set->size < (1LL << 30);
 }
 
-// the order the flux pass takes these edges in; nullptr: the loop's own
-static const SlotPlan::Order *flux_order(SlotPlan *sp, const op_arg *ra) {
-  if (!tuning("flux_order", 1) || !tuning("flux_pair", 1) ||
-      !flux_pair_shape(ra, (size_t)sp->na + sp->nb + 1))
+// the order the flux pass takes these edges in; nullptr: the loop's own.  next:
+// a pass is about to run, and may be the first in an order made for it.  Making
+// one costs what it saves in about 4 + 6M / edges passes (100 us and 17 us a
+// pass and million edges), so a mesh evaluated a few times does without: the
+// first nine evaluations of 21k cells in FP64 took 747 us with it, 649 without.
+// A million edges and more start with it, since ten passes are five iterations:
+// the first four of 2.88M cells 3.72 ms, 4.02 without it, 4.20 from the sixth
+// pass on.
+static const SlotPlan::Order *flux_order(SlotPlan *sp, const op_arg *ra, bool next) {
+  const int on = sp->scattered ? tuning("flux_order", 1) : 0;
+  if (!on || !tuning("flux_pair", 1) || !flux_pair_shape(ra, (size_t)sp->na + sp->nb + 1))
     return nullptr;
-  return get_flux_order(sp, ra[0].map, ra[2].map, ra[0].dat);
+  const long long after = on == 2 || sp->na >= 1 << 20 ? 0 : 4 + 6000000 / std::max(sp->na, 1);
+  return get_flux_order(sp, ra[0].map, ra[2].map, ra[0].dat, next ? after : -1);
 }
 
 // the flux pass of res_calc (and bres_calc's values when B.n > 0) into vals
@@ -1879,7 +1887,7 @@ static void launch_flux(SlotPlan *sp, const op_arg *ra, const ResEdges<T> &E,
   if (per_sm > 0) fg = std::min(fg, (long long)rt().num_sms * per_sm);
   const unsigned fgrid = (unsigned)std::max(1LL, fg);
   if (flux_pair_shape(ra, nval) && tuning("flux_pair", 1)) {
-    const SlotPlan::Order *o = flux_order(sp, ra);
+    const SlotPlan::Order *o = flux_order(sp, ra, false);
     const RedTail<T> tail = red_tail_take<T>();
     launch_pdl(o ? k_res_flux_pair<T, true> : k_res_flux_pair<T, false>,
                fgrid + (tail.n ? 1 : 0), 256, 0, s, E.n, (const int4 *)(o ? o->d_rows : nullptr),
@@ -2093,6 +2101,8 @@ static bool res_flux_ahead_t(op_set rset, const op_arg *ra, op_set bset, const o
   if (ra[4].dat == adt) E.adta = (const T *)adt_now;
   if (ra[5].dat == adt) E.adtb = (const T *)adt_now;
   if (ba && ba[3].dat == adt) B.adt = (const T *)adt_now;
+  flux_order(sp, ra, true);
+  if (error_pending()) return false;
   launch_flux<T>(sp, ra, E, B, (T *)sp->d_buf, (size_t)sp->na + sp->nb + 1, K, rt().stream);
   return true;
 }
@@ -2687,7 +2697,7 @@ static bool res_chain_t(char const *loop_name, op_set rset, const op_arg *ra, op
   T *vals = (T *)sp->d_buf;
   const bool col = effective_strategy(key.rname) == OP2B_STRATEGY_COLOURED;
   // the lists that go with the flux pass's order
-  const SlotPlan::Order *order = flux_order(sp, ra);
+  const SlotPlan::Order *order = flux_order(sp, ra, !flux_done);
   if (error_pending()) return true;
   const int *ell = order ? order->d_ell : sp->d_ell;
   if (col) {

@@ -124,6 +124,7 @@ int op2b_capture_begin(int profile) {
   flush_pending();  // loops held back before the capture run outside the graph
   red_tail_flush();
   ahead_drop();     // a graph bakes dataset pointers: nothing may be swapped in later
+  make_flux_orders();
   tile_capture_begin();
   known_zero_capture_begin();
   g_capture_zero_entries.clear();

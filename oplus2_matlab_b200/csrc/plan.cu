@@ -1957,21 +1957,14 @@ static bool coord_order(int na, int nnode, const int2 *edge, const int2 *cell, c
   return true;
 }
 
-const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq, op_dat x) {
-  if (!sp->scattered) return nullptr;
-  for (auto &o : sp->orders)
-    if (o->mx == mx && o->mq == mq) return o->d_rows ? o.get() : nullptr;
+static void make_flux_order(SlotPlan *sp, SlotPlan::Order *o) {
   cudaStream_t s = rt().stream;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  OP2B_CUDA(cudaStreamIsCapturing(s, &cap));
-  if (cap != cudaStreamCaptureStatusNone) return nullptr;
+  const op_dat x = o->x;
   const int na = sp->na, nchunk = (na + kOrderChunk - 1) / kOrderChunk;
-  const int2 *edge = reinterpret_cast<const int2 *>(map_dev(mx));
-  const int2 *cell = reinterpret_cast<const int2 *>(map_dev(mq));
+  const int2 *edge = reinterpret_cast<const int2 *>(map_dev(o->mx));
+  const int2 *cell = reinterpret_cast<const int2 *>(map_dev(o->mq));
   const size_t nlist = (size_t)sp->width * sp->ntarget;
-  std::unique_ptr<SlotPlan::Order> o(new SlotPlan::Order());
-  o->mx = mx;
-  o->mq = mq;
+  o->tried = true;
   o->d_rows = (int4 *)dev_try_alloc(sizeof(int4) * (size_t)na + sizeof(int) * nlist);
   o->d_ell = (int *)(o->d_rows + (o->d_rows ? na : 0));
   // edges' places | distinct cells of a sample of the new order, of the old
@@ -2000,8 +1993,39 @@ const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq, op_dat
     o->d_ell = nullptr;
   }
   if (mem) OP2B_CUDA(cudaFreeAsync(mem, s));
-  sp->orders.push_back(std::move(o));
-  return sp->orders.back()->d_rows ? sp->orders.back().get() : nullptr;
+  if (!o->d_rows) return;
+  const std::vector<SlotPlan::Coloured> had = sp->coloured;
+  for (const auto &c : had)
+    if (!c.o) get_coloured_lists(sp, o, c.p, c.nt, c.pb, c.nbt);
+}
+
+const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq, op_dat x,
+                                      long long after) {
+  if (!sp->scattered) return nullptr;
+  SlotPlan::Order *o = nullptr;
+  for (auto &p : sp->orders)
+    if (p->mx == mx && p->mq == mq) o = p.get();
+  if (o && (o->d_rows || o->tried)) return o->d_rows ? o : nullptr;
+  if (after < 0) return nullptr;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  OP2B_CUDA(cudaStreamIsCapturing(rt().stream, &cap));
+  if (cap != cudaStreamCaptureStatusNone) return nullptr;
+  if (!o) {
+    sp->orders.emplace_back(new SlotPlan::Order());
+    o = sp->orders.back().get();
+    o->mx = mx;
+    o->mq = mq;
+  }
+  o->x = x;
+  if (o->passes++ < after) return nullptr;
+  make_flux_order(sp, o);
+  return o->d_rows ? o : nullptr;
+}
+
+void make_flux_orders() {
+  for (auto &sp : g_slot_plans)
+    for (auto &o : sp->orders)
+      if (!o->d_rows && !o->tried) make_flux_order(sp.get(), o.get());
 }
 
 }  // namespace op2b

@@ -94,9 +94,12 @@ struct SlotPlan {
   bool chain_unsuited = false;  // a cell tile reads too many flux tiles for it
   // the edges of a in the order the flux pass takes them (get_flux_order)
   struct Order {
-    op_map mx, mq;          // the maps of the edges' nodes and cells
-    int4 *d_rows;           // [na] the edges' rows of them: two nodes, two cells
-    int *d_ell;             // the lists, with the places of the edges' values
+    op_map mx = nullptr, mq = nullptr;  // the maps of the edges' nodes and cells
+    op_dat x = nullptr;                 // the nodes' coordinates
+    int4 *d_rows = nullptr;  // [na] the edges' rows of them: two nodes, two cells
+    int *d_ell = nullptr;    // the lists, with the places of the edges' values
+    long long passes = 0;    // flux passes in the loop's order
+    bool tried = false;
   };
   std::vector<std::unique_ptr<Order>> orders;
   bool scattered = false;  // a's elements, in order, reach targets without locality
@@ -126,7 +129,13 @@ const int *get_coloured_lists(SlotPlan *sp, const SlotPlan::Order *o, const DevP
 // columns 0 and 1 of the dim-2 maps mx and mq and whose nodes have the dataset
 // x (two reals: taken for coordinates when the numbering has no locality);
 // nullptr: the loop's own order, or a capture that comes before it is built.
-const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq, op_dat x);
+// after: the order may be made now, if this is at least that many passes after
+// the first; < 0: only one that is there.  Values of a flux pass that has run are
+// listed in the order that it took, so only a caller about to run one may make it
+const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq, op_dat x,
+                                      long long after);
+// at the start of a capture, which is replayed often and cannot make them
+void make_flux_orders();
 
 // widest list the fold kernels accept
 constexpr int kMaxSlotWidth = 8;
