@@ -14,7 +14,7 @@
  * and a solve's first ones in a launch before its first iteration.  The per-element arithmetic is the plain path's
  * (same device functions, same contribution order), so a solve's flow field
  * q is bit-identical to the plain op_par_loop solve of the same mesh and
- * flow.  Each solve's rms is folded from its own tiles' partials, in tile
+ * flow.  Each solve's rms is folded from partials of 256 consecutive cells, in
  * order, by the last of its CTAs to finish: it depends only on that solve, so
  * a solve's results are bit-identical whether it runs alone or with any
  * other solves.  The rms history and the stopping test live on the device:
