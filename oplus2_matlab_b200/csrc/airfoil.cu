@@ -659,8 +659,9 @@ __global__ void __launch_bounds__(256, MINB)
 // ahead, so a warp has a cell's loads in flight while it computes.
 // Bound: the latency of the gathers (ten of the eighteen cycles a warp spends
 // per instruction in the general form).  Registers pay for the loads in
-// flight, not for warps: 2 CTAs of 256 per SM (FP64 1) beat 3 and 4, which
-// spill (iteration 47.1 against 55.4 and 63.6 us at 720k FP32), and 128-thread
+// flight, not for warps: at least 2 CTAs of 256 per SM (FP64 1; without
+// adt_calc and res FP32 fits 3) beat bounds of 3 and 4, which spill with
+// adt_calc (iteration 47.1 against 55.4 and 63.6 us at 720k FP32), and 128-thread
 // CTAs, whose partials take longer to fold (48.0).  Against the general form:
 // 49.1 -> 47.1 us an iteration at 720k FP32, 57.3 -> 54.1 at 407k FP64.
 template <class T>
@@ -2806,17 +2807,20 @@ static bool res_chain_t(char const *loop_name, op_set rset, const op_arg *ra, op
         auto kernel = skip_res ? ks : kr;
         const bool leave = !seq && red_tail_wanted(tail_next);
         if (!leave && !seq) rslot.seq = tail_seq = red_flag(rslot_id, &rslot.flag);
-        launch_pdl(kernel, grid_of((const void *)kernel, kFoldThreads), kFoldThreads, 0, s, (unsigned)ncell,
+        // one grid for both kernels: a graph launch that puts kr in place of
+        // ks leaves as many partials as the kernel that folds them was told
+        // (ks may fit more CTAs per SM: FP32 without adt_calc 80 registers and
+        // 3 of them, kr 94 and 2)
+        const int grid = grid_of((const void *)kernel, kFoldThreads);
+        launch_pdl(kernel, grid, kFoldThreads, 0, s, (unsigned)ncell,
                    reinterpret_cast<const int4 *>(ell), (const T *)vals, qold, q,
                    skip_res ? (T *)nullptr : res, (const T *)adt,
                    reinterpret_cast<const int4 *>(N.m0.map), xs[0], K, seqbuf, rslot,
                    leave ? nullptr : red_ticket(), qsave, adt_to ? adt_to : adt);
         if (skip_res)
-          zero_entry(ra[6].dat, 5, kernel_nparams(kernel), (const void *)kr,
-                     grid_of((const void *)kr, kFoldThreads));
+          zero_entry(ra[6].dat, 5, kernel_nparams(kernel), (const void *)kr, grid);
         if (leave)
-          tail_seq = red_tail_leave(sizeof(T) == 8 ? GBL_F64 : GBL_F32,
-                                    grid_of((const void *)kernel, kFoldThreads), rslot_id, -1, 12,
+          tail_seq = red_tail_leave(sizeof(T) == 8 ? GBL_F64 : GBL_F32, grid, rslot_id, -1, 12,
                                     kernel_nparams(kernel));
       };
 #define OP2B_CELLS(ADT, SAVE, COL) \
