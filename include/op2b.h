@@ -71,7 +71,9 @@ enum { OP2B_REDUCE_TREE = 0, OP2B_REDUCE_SEQ = 1 };
  *                   from the pass on by which making the order pays, or a
  *                   capture; 2: from the first pass; 0: in edge order
  *   "red_tail"      1 (default): the rms of an update is folded by the flux
- *                   pass behind it; 0: by the update's last block
+ *                   pass behind it, where the library issues that one too
+ *                   (run ahead, or in a capture by op2b_capture_begin); 0: by
+ *                   the update's last block
  *   "coloured_fold" 1 (default): COLOURED res_calc [+ bres_calc ...] as the
  *                   flux pass and a per-cell fold in the plan's order; 0: one
  *                   launch per block colour

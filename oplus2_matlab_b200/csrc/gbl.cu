@@ -150,12 +150,7 @@ unsigned red_flag(int slot, unsigned **flag) {
 }
 
 bool red_tail_wanted(bool tail_next) {
-  if (!tuning("red_tail", 1)) return false;
-  if (!rt().gbl_deferred) return tail_next;
-  if (rt().own_capture) return true;
-  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  OP2B_CUDA(cudaStreamIsCapturing(rt().stream, &st));
-  return st == cudaStreamCaptureStatusNone;
+  return tuning("red_tail", 1) && (rt().gbl_deferred ? rt().own_capture : tail_next);
 }
 
 unsigned red_tail_leave(int type, int n, int slot, int slot_max, int ticket_arg, int nparams) {

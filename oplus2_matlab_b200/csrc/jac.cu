@@ -333,8 +333,8 @@ static void jac_update_t(char const *name, op_set set, const op_arg *args,
     LoopScope ls(name, compulsory_bytes(set, 5, args), 0);
     float *seqbuf = seq ? (float *)red_seq_buffer(sizeof(float) * (size_t)n) : nullptr;
     const int threads = 256, grid = red_grid(n, threads);
-    // the sum and the maximum are left to the res that follows, at once or,
-    // with deferred reductions, in all likelihood
+    // the sum and the maximum are left to the res that follows at once, or in
+    // the library's own capture
     const bool leave = !seq && red_tail_wanted(tail_next);
     RedSlot<float> ss{(float *)red_partials(0), r_sum}, sm{(float *)red_partials(1), r_max};
     if (!leave && !seq) ss.seq = flag_seq = red_flag(slot_sum, &ss.flag);

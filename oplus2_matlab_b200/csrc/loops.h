@@ -64,7 +64,12 @@ unsigned seq_sum(const T *v, long long n, T init, T *out, const int *order, int 
 // the kernel's parameter that makes it fold its partials itself, given a
 // ticket (of nparams parameters), for a capture that ends before another
 // kernel takes the tail.
-// Not in a caller's own stream capture, which ends without the library.
+// Only where the fold is sure to be issued by the library on the same stream:
+// inside its own capture (which patches what is left at the end), or, with
+// tail_next, by the call that leaves it.  Never with deferred reductions
+// outside a capture: what comes next may be a capture of the caller's, which
+// would record the fold and not run it, or a graph of the caller's, whose
+// updates write the same partials.
 bool red_tail_wanted(bool tail_next);
 unsigned red_tail_leave(int type, int n, int slot, int slot_max, int ticket_arg, int nparams);
 template <class T>

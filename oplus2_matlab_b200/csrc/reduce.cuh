@@ -123,8 +123,9 @@ __device__ __forceinline__ void grid_leave(const T (&v)[N], const T (&identity)[
 // waiting for a chain of fence, ticket, loads and a store to host memory
 // (2 us at the end of every res_calc chain: 47.2 -> 45.2 us a captured
 // iteration of 720k FP32 cells with one of its two chains relieved, 14.4 -> 12.4
-// at 7k); a CTA of the next kernel does it while the others work.  flag, when not null, is set to seq once the results
-// are in host memory, for a host that waits for them.
+// at 7k); a CTA of the next kernel does it while the others work.  flag, when
+// not null, is set to seq once the results are in host memory, for a host that
+// waits for them.
 template <class T>
 struct RedTail {
   const T *sums, *maxs;  // [n]; maxs may be null

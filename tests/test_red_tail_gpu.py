@@ -2,6 +2,8 @@
 number of block partials or the place of the fold could go wrong.  With the
 knob at 0 each update folds its own partials in the same order, so every rms
 must be equal bit for bit."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -67,3 +69,96 @@ def test_graph_launched_when_res_is_not_zero(op2, dt, strategy):
     api.op_exit()
     api.op_init([], 0)
     assert run(1) == want
+
+
+def cudart():
+    for name in ("libcudart.so.12", "libcudart.so"):
+        try:
+            rt = C.CDLL(name)
+            break
+        except OSError:
+            continue
+    P = C.c_void_p
+    rt.cudaStreamBeginCapture.argtypes = [P, C.c_int]
+    rt.cudaStreamEndCapture.argtypes = [P, C.POINTER(P)]
+    rt.cudaGraphDestroy.argtypes = [P]
+    return rt
+
+
+RELAXED = 2  # cudaStreamCaptureModeRelaxed
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+def test_a_callers_capture_records_no_fold_of_an_earlier_update(op2, dt):
+    """A deferred update, then a stream capture of the caller's own (never
+    launched) of loops whose flux pass could take the update's rms along:
+    op2b_sync delivers the rms all the same."""
+    mesh = M.naca0012(41, 61)
+    rt = cudart()
+
+    def run(tail, capture):
+        A = start(mesh, dt, api.STRATEGY_GATHER, tail)
+        A.iterate(2)
+        for nm in ("adt_calc", "res_calc", "bres_calc", "adt_calc"):  # plans without update
+            A.loop(nm)
+        A.iterate(1)
+        api.set_gbl_deferred(1)
+        A.rms[0] = 0
+        for nm in ("save_soln", "adt_calc") + STAGE + ("adt_calc",):
+            A.loop(nm)  # the last call runs the held update
+        if capture:
+            s = C.c_void_p(api.get_stream())
+            assert rt.cudaStreamBeginCapture(s, RELAXED) == 0
+            for nm in ("res_calc", "bres_calc", "adt_calc"):
+                A.loop(nm)
+            g = C.c_void_p()
+            assert rt.cudaStreamEndCapture(s, C.byref(g)) == 0
+            assert rt.cudaGraphDestroy(g) == 0
+        api.sync()
+        assert api.last_error() == ""
+        return float(A.rms[0])
+
+    want = run(0, False)
+    assert want > 0
+    for tail, capture in ((1, False), (0, True), (1, True)):
+        api.set_gbl_deferred(0)
+        api.op_exit()
+        api.op_init([], 0)
+        assert run(tail, capture) == want, (tail, capture)
+
+
+def test_a_jac_update_before_a_callers_capture(op2):
+    """The same with jac1's sum and maximum and the res behind them."""
+    rt = cudart()
+
+    def run(tail, capture):
+        api.set_strategy(api.STRATEGY_GATHER)
+        api.lib().op2b_set_tuning(b"red_tail", tail)
+        api.lib().op2b_set_tuning(b"jac_step", 0)
+        J = apps.Jac(M.jac(40, 1), 1)
+        J.iterate(2)
+        api.set_gbl_deferred(1)
+        api.op_par_loop("res", J.edges, *J.res_args)
+        J.u_sum[0] = J.u_max[0] = 0
+        api.op_par_loop("update", J.nodes, *J.upd_args)
+        if capture:
+            s = C.c_void_p(api.get_stream())
+            assert rt.cudaStreamBeginCapture(s, RELAXED) == 0
+            api.op_par_loop("res", J.edges, *J.res_args)
+            g = C.c_void_p()
+            assert rt.cudaStreamEndCapture(s, C.byref(g)) == 0
+            assert rt.cudaGraphDestroy(g) == 0
+        api.sync()
+        assert api.last_error() == ""
+        return float(J.u_sum[0]), float(J.u_max[0])
+
+    try:
+        want = run(0, False)
+        assert want[0] > 0
+        for tail, capture in ((1, False), (0, True), (1, True)):
+            api.set_gbl_deferred(0)
+            api.op_exit()
+            api.op_init([], 0)
+            assert run(tail, capture) == want, (tail, capture)
+    finally:
+        api.lib().op2b_set_tuning(b"jac_step", 1)
