@@ -224,6 +224,11 @@ void red_tail_patch_captured() {
   g_tail_patches.clear();
 }
 
+void red_tail_drop_captured() {
+  g_tail_patches.clear();
+  if (g_tail.captured) g_tail.on = false;
+}
+
 // every reduction asks for its partials before it is launched: those of the
 // one before it are folded by then
 void *red_partials(int i) {

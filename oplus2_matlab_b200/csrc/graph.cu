@@ -162,6 +162,7 @@ void *op2b_capture_end(void) {
   g->reductions = red_take_pending_since(g_pending_mark);
   red_reserve_for_graph();
   if (e != cudaSuccess) {
+    red_tail_drop_captured();
     delete g;
     fail(-1, "op2b error: graph capture failed: %s\n", cudaGetErrorString(e));
     return nullptr;

@@ -79,6 +79,8 @@ RedTail<T> red_tail_take();  // n == 0: none, or of the other type
 void red_tail_flush();
 // at the end of a capture: the kernels that now fold their own partials
 void red_tail_patch_captured();
+// after a capture that failed: nothing of its graph, which is gone, is kept
+void red_tail_drop_captured();
 void red_finish(const std::vector<GblRequest> &reqs);
 // the same, waiting only for the work up to the event, or for the requests'
 // flags when they have them (not deferred mode)

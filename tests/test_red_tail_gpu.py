@@ -82,6 +82,7 @@ def cudart():
     rt.cudaStreamBeginCapture.argtypes = [P, C.c_int]
     rt.cudaStreamEndCapture.argtypes = [P, C.POINTER(P)]
     rt.cudaGraphDestroy.argtypes = [P]
+    rt.cudaStreamSynchronize.argtypes = [P]
     return rt
 
 
@@ -162,3 +163,54 @@ def test_a_jac_update_before_a_callers_capture(op2):
             assert run(tail, capture) == want, (tail, capture)
     finally:
         api.lib().op2b_set_tuning(b"jac_step", 1)
+
+
+def test_a_capture_after_one_that_failed(op2):
+    """jac1's update twice in a capture: the second has the first fold its own
+    partials, which is put into the graph at the capture's end.  A
+    synchronisation breaks the capture before that; the next capture holds
+    nothing of it and its sums are those of the loops."""
+    rt, lib = cudart(), api.lib()
+
+    def run(failed, tail):
+        lib.op2b_set_tuning(b"red_tail", tail)
+        lib.op2b_set_tuning(b"jac_step", 0)
+        J = apps.Jac(M.jac(40, 1), 1)
+        J.iterate(2)
+
+        def update():
+            api.op_par_loop("update", J.nodes, *J.upd_args)
+
+        if failed:
+            assert lib.op2b_capture_begin(0) == 1
+            update()
+            update()
+            assert rt.cudaStreamSynchronize(C.c_void_p(api.get_stream())) != 0
+            assert not lib.op2b_capture_end()
+            assert "capture failed" in api.last_error()
+            api.clear_error()
+        assert lib.op2b_capture_begin(0) == 1
+        api.op_par_loop("res", J.edges, *J.res_args)
+        update()
+        api.op_par_loop("res", J.edges, *J.res_args)
+        update()
+        h = lib.op2b_capture_end()
+        assert h, api.last_error()
+        out = []
+        for _ in range(3):
+            J.u_sum[0] = J.u_max[0] = 0
+            assert lib.op2b_graph_launch(h) == 0
+            api.sync()
+            out.append((float(J.u_sum[0]), float(J.u_max[0])))
+        lib.op2b_graph_destroy(h)
+        assert api.last_error() == ""
+        return out
+
+    try:
+        want = run(False, 0)
+        for failed, tail in ((True, 1), (False, 1)):
+            api.op_exit()
+            api.op_init([], 0)
+            assert run(failed, tail) == want
+    finally:
+        lib.op2b_set_tuning(b"jac_step", 1)
