@@ -2011,22 +2011,24 @@ static ChainSched *chain_sched(SlotPlan *sp, int et, int ct, int lag) {
 }
 
 // the plans and value buffer of a res_calc (+ bres_calc) chain; nullptr
-// when the mesh does not suit slots; *err when a plan failed
+// when the mesh does not suit slots, or when something is not there yet and
+// build is false; *err when a plan failed
 template <class T>
 static SlotPlan *chain_plans(op_set rset, const op_arg *ra, op_set bset, const op_arg *ba,
-                             bool *err) {
+                             bool *err, bool build = true) {
   *err = false;
-  GatherPlan *g = get_gather_plan(rset, ra, {6, 7});
-  GatherPlan *gb = ba ? get_gather_plan(bset, ba, {4}) : nullptr;
+  GatherPlan *g = get_gather_plan(rset, ra, {6, 7}, build);
+  GatherPlan *gb = ba ? get_gather_plan(bset, ba, {4}, build) : nullptr;
   if (!g || (ba && !gb)) {
-    *err = true;
+    *err = build;
     return nullptr;
   }
-  SlotPlan *sp = get_slot_plan(g, gb);
+  SlotPlan *sp = get_slot_plan(g, gb, build);
   if (!sp) return nullptr;
   const size_t nval = (size_t)sp->na + sp->nb + 1;
   const size_t need = sizeof(T) * 4 * nval;
   if (sp->buf_bytes < need) {
+    if (!build) return nullptr;
     dev_free(sp->d_buf);
     sp->d_buf = dev_alloc(need);
     sp->buf_bytes = sp->d_buf ? need : 0;
@@ -2051,7 +2053,8 @@ static SlotPlan *chain_plans(op_set rset, const op_arg *ra, op_set bset, const o
 // block colours, each launch a chain of dependent steps over a quarter of the
 // blocks; 116 us so.
 // The block kernels remain for cells of more than kMaxSlotWidth
-// contributions and for bres_calc on its own.
+// contributions, for bres_calc on its own, and in a capture of a loop whose
+// lists are not there yet.
 bool coloured_fold() { return tuning("coloured_fold", 1) && tuning("gather_slots", 1); }
 
 static const int *coloured_ell(SlotPlan *sp, const SlotPlan::Order *o, op_set rset,
@@ -2690,13 +2693,15 @@ static bool res_chain_t(char const *loop_name, op_set rset, const op_arg *ra, op
   if (error_pending()) return true;
   cudaStream_t s = rt().stream;
   bool err = false;
-  SlotPlan *sp = chain_plans<T>(rset, ra, bset, ba, &err);
+  const bool col = effective_strategy(key.rname) == OP2B_STRATEGY_COLOURED;
+  // a capture cannot make plans: COLOURED runs by block colours there unless
+  // all that its two passes need is there
+  SlotPlan *sp = chain_plans<T>(rset, ra, bset, ba, &err, !col || !stream_capturing());
   if (err) return true;
   if (!sp) return false;
   const int W = sp->width, ncell = sp->ntarget;
   const size_t nval = (size_t)sp->na + sp->nb + 1;
   T *vals = (T *)sp->d_buf;
-  const bool col = effective_strategy(key.rname) == OP2B_STRATEGY_COLOURED;
   // the lists that go with the flux pass's order
   const SlotPlan::Order *order = flux_order(sp, ra, !flux_done);
   if (error_pending()) return true;

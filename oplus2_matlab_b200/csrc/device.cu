@@ -81,6 +81,7 @@ cudaMemPool_t g_pool = nullptr;
 int g_pool_device = -1;
 bool g_pool_off = false, g_pool_checked = false;
 std::unordered_set<void *> g_pooled;  // live buffers that came from the pool
+}  // namespace
 
 bool stream_capturing() {
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
@@ -91,6 +92,7 @@ bool stream_capturing() {
   return st != cudaStreamCaptureStatusNone;
 }
 
+namespace {
 cudaMemPool_t pool() {
   if (!g_pool_checked) {
     const char *e = getenv("OP2B_POOL");

@@ -134,6 +134,9 @@ void flush_pending();
 // device memory helpers (long-lived allocations)
 void *dev_alloc(size_t bytes);
 void *dev_try_alloc(size_t bytes);  // nullptr and no error when there is no room
+// a capture of the library's stream is under way, the library's own or the
+// caller's: what is launched now is recorded, not run
+bool stream_capturing();
 void dev_free(void *p);
 // stream-ordered scratch from the library's pool; free with cudaFreeAsync
 cudaError_t pool_malloc_async(void **p, size_t bytes, cudaStream_t s);

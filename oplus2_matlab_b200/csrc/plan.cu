@@ -1508,7 +1508,8 @@ __global__ void k_keys_through(int *keys, long long n, int nslots, const int *pe
   }
 }
 
-GatherPlan *get_gather_plan(op_set set, const op_arg *args, const std::vector<int> &slots) {
+GatherPlan *get_gather_plan(op_set set, const op_arg *args, const std::vector<int> &slots,
+                            bool build) {
   for (auto &up : g_gather) {
     GatherPlan &g = *up;
     if (g.set != set || g.nslots != (int)slots.size() || g.dat != args[slots[0]].dat) continue;
@@ -1517,6 +1518,7 @@ GatherPlan *get_gather_plan(op_set set, const op_arg *args, const std::vector<in
       match = g.maps[k] == args[slots[k]].map && g.idxs[k] == args[slots[k]].idx;
     if (match) return &g;
   }
+  if (!build) return nullptr;
   Runtime &R = rt();
   cudaStream_t s = R.stream;
   std::unique_ptr<GatherPlan> up(new GatherPlan());
@@ -1674,9 +1676,10 @@ __global__ void __launch_bounds__(kOrderChunk)
 
 static std::vector<std::unique_ptr<SlotPlan>> g_slot_plans;
 
-SlotPlan *get_slot_plan(const GatherPlan *a, const GatherPlan *b) {
+SlotPlan *get_slot_plan(const GatherPlan *a, const GatherPlan *b, bool build) {
   for (auto &up : g_slot_plans)
     if (up->a == a && up->b == b) return up->width > 0 ? up.get() : nullptr;
+  if (!build) return nullptr;
   std::unique_ptr<SlotPlan> up(new SlotPlan());
   SlotPlan &p = *up;
   p.a = a;
@@ -1783,7 +1786,7 @@ const int *get_coloured_lists(SlotPlan *sp, const SlotPlan::Order *o, const DevP
                               const DevPlan *pb, int nbt) {
   for (auto &c : sp->coloured)
     if (c.o == o && c.p == p && c.pb == pb && c.nt == nt && c.nbt == nbt) return c.d_ell;
-  if ((long long)sp->na + sp->nb + 1 >= (1LL << 29)) return nullptr;
+  if ((long long)sp->na + sp->nb + 1 >= (1LL << 29) || stream_capturing()) return nullptr;
   SlotPlan::Coloured c{p, pb, o, nt, nbt, nullptr};
   c.d_ell = (int *)dev_alloc(sizeof(int) * (size_t)sp->width * sp->ntarget);
   if (!c.d_ell) return nullptr;
@@ -2006,10 +2009,7 @@ const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq, op_dat
   for (auto &p : sp->orders)
     if (p->mx == mx && p->mq == mq) o = p.get();
   if (o && (o->d_rows || o->tried)) return o->d_rows ? o : nullptr;
-  if (after < 0) return nullptr;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  OP2B_CUDA(cudaStreamIsCapturing(rt().stream, &cap));
-  if (cap != cudaStreamCaptureStatusNone) return nullptr;
+  if (after < 0 || stream_capturing()) return nullptr;
   if (!o) {
     sp->orders.emplace_back(new SlotPlan::Order());
     o = sp->orders.back().get();
@@ -2023,6 +2023,7 @@ const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq, op_dat
 }
 
 void make_flux_orders() {
+  if (stream_capturing()) return;
   for (auto &sp : g_slot_plans)
     for (auto &o : sp->orders)
       if (!o->d_rows && !o->tried) make_flux_order(sp.get(), o.get());

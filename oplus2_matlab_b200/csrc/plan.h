@@ -121,7 +121,8 @@ void release_tile_plan(SlotPlan *sp);
 // strip of nt elements of the block, thread colour and slot, b's after a's;
 // entry index << 2 | last of its block << 1 | negate, -1 past the end.
 // o: when the flux pass has an order of its own.
-// Device memory kept with the slot plan; nullptr when the indices do not fit.
+// Device memory kept with the slot plan; nullptr when the indices do not fit, or
+// when they are not there and a capture is under way, which cannot make them.
 const int *get_coloured_lists(SlotPlan *sp, const SlotPlan::Order *o, const DevPlan *p, int nt,
                               const DevPlan *pb, int nbt);
 
@@ -144,14 +145,16 @@ constexpr int kMaxSlotWidth = 8;
 // nullptr when some target has more than kMaxSlotWidth contributions or the
 // padding would more than double the lists (the caller then uses the CSR
 // fold).
-SlotPlan *get_slot_plan(const GatherPlan *a, const GatherPlan *b);
+// (build false, here and for get_gather_plan: nullptr if it is not there yet)
+SlotPlan *get_slot_plan(const GatherPlan *a, const GatherPlan *b, bool build = true);
 
 // Find or build the reference-compatible plan (device resident).
 DevPlan *get_plan(char const *name, op_set set, int part_size, int nargs, const op_arg *args,
                   int ninds, const int *inds);
 // Find or build the gather plan for the INC args listed in slots (all on
 // the same dat).
-GatherPlan *get_gather_plan(op_set set, const op_arg *args, const std::vector<int> &slots);
+GatherPlan *get_gather_plan(op_set set, const op_arg *args, const std::vector<int> &slots,
+                            bool build = true);
 // Device validation of a plan; returns the number of violations.
 long validate_plan(const DevPlan &p);
 
