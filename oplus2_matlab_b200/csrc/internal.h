@@ -93,6 +93,9 @@ struct Runtime {
   // into the graph when profiling
   bool capture_profile = false;
   bool own_capture = false;  // between op2b_capture_begin and op2b_capture_end
+  // kernels that write plan arrays were queued on the stream and no kernel
+  // that reads them yet (launch_pdl)
+  bool plan_queued = false;
   struct CapturedLoop {
     std::string name;
     cudaEvent_t start, stop;

@@ -239,6 +239,7 @@ static int2 *jac_pairs(const GatherPlan *g, const op_arg *args, cudaStream_t s) 
   if (g->nkeys)
     k_jac_pairs<<<rt().num_sms * 8, 256, 0, s>>>(g->nkeys, g->d_keys, idx_map(args[0]),
                                                  idx_map(args[1]), p.d);
+  rt().plan_queued = true;
   g_jac_pairs.push_back(p);
   return p.d;
 }

@@ -12,8 +12,14 @@
 //      may take the SM slots this grid frees.
 // A kernel triggers only after its own wait, so when the next kernel starts
 // every kernel before this one has completed.  Without the attribute (the
-// "pdl" tuning knob at 0), or after a kernel that never triggers, both
-// instructions are no-ops and ordering is the stream's usual one.
+// "pdl" tuning knob at 0) both instructions are no-ops and ordering is the
+// stream's usual one.
+// Step 1 is not ordered with the launch directly in front: that one may have
+// ended, but only the wait promises that what it wrote is visible.  So what
+// fills a plan array without a host wait behind it sets rt().plan_queued, and
+// the next launch on the stream goes without the attribute, after everything
+// before it; the one behind that may read early again, since the launch
+// between has waited.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -51,6 +57,10 @@ inline void launch_pdl(void (*kernel)(KArgs...), unsigned grid, unsigned block, 
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = tuning("pdl", 1) ? 1 : 0;
+  if (s == rt().stream && rt().plan_queued) {
+    rt().plan_queued = false;
+    cfg.numAttrs = 0;
+  }
   OP2B_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...));
 }
 

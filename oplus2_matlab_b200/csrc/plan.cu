@@ -1797,6 +1797,7 @@ const int *get_coloured_lists(SlotPlan *sp, const SlotPlan::Order *o, const DevP
                                                               sp->nb, sp->d_ell,
                                                               o ? o->d_ell : sp->d_ell, A, B,
                                                               c.d_ell);
+  rt().plan_queued = true;
   sp->coloured.push_back(c);
   return c.d_ell;
 }
@@ -1989,6 +1990,7 @@ static void make_flux_order(SlotPlan *sp, SlotPlan::Order *o) {
     k_chunk_cells<<<nsample, kOrderChunk, 0, s>>>(step, na, cell, nullptr, cells + 1);
     k_order_lists<<<rt().num_sms * 8, 256, 0, s>>>(nlist, na, sp->d_ell, mem, cells, edge, cell,
                                                    o->d_rows, o->d_ell);
+    rt().plan_queued = true;
   } else {
     cudaGetLastError();
     dev_free(o->d_rows);
