@@ -233,6 +233,7 @@ static int2 *jac_pairs(const GatherPlan *g, const op_arg *args, cudaStream_t s) 
     if (p.g == g && p.mA == args[0].map && p.mu == args[1].map && p.iA == args[0].idx &&
         p.iu == args[1].idx)
       return p.d;
+  if (stream_capturing()) return nullptr;  // recorded, they would not be there for other calls
   JacPairs p{g, args[0].map, args[1].map, args[0].idx, args[1].idx, nullptr};
   p.d = (int2 *)dev_alloc(sizeof(int2) * (size_t)std::max(1LL, g->nkeys));
   if (!p.d) return nullptr;

@@ -77,6 +77,42 @@ def test_first_pass_of_a_rejected_order(dt):
 
 
 @pytest.mark.parametrize("variant", [1, 2])
+def test_pairs_are_not_made_in_a_capture(variant):
+    """A capture's first res through another column of the map, then the same
+    loop outside before the graph is launched; against the loop alone."""
+    mesh = M.jac(100, variant)
+
+    def run(capture):
+        lib = api.lib()
+        api.set_strategy(api.STRATEGY_GATHER)
+        J = apps.Jac(mesh, variant)
+        J.iterate(2)
+        args = list(J.res_args)
+        args[1] = api.op_arg_dat(J.p_u, 0, J.ppedge, J.u.shape[1], "float", api.OP_READ)
+        if capture:
+            assert lib.op2b_capture_begin(0) == 1, api.last_error()
+            api.op_par_loop("res", J.edges, *args)
+            h = lib.op2b_capture_end()
+            assert h, api.last_error()
+        api.op_par_loop("res", J.edges, *args)
+        if capture:
+            assert lib.op2b_graph_launch(h) == 0
+            api.sync()
+            lib.op2b_graph_destroy(h)
+        else:
+            api.op_par_loop("res", J.edges, *args)
+        api.op_fetch_data(J.p_du)
+        assert api.last_error() == ""
+        return J.du.copy()
+
+    want = run(False)
+    api.op_exit()
+    api.op_init([], 0)
+    assert np.any(want != 0)
+    assert run(True).tobytes() == want.tobytes()
+
+
+@pytest.mark.parametrize("variant", [1, 2])
 def test_first_res_of_jac(variant):
     mesh = M.jac(200, variant)
 
