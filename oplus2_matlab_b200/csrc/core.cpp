@@ -11,6 +11,7 @@
 #include <thread>
 #include <vector>
 
+#include "host_threads.h"
 #include "internal.h"
 
 extern "C" {
@@ -164,16 +165,12 @@ static unsigned range_check(const int *imap, size_t n, unsigned lim) {
   const size_t nt = n < ((size_t)1 << 20) || hw < 2 ? 1 : std::min<size_t>(8, hw);
   if (nt == 1) return part(0, n);
   std::vector<unsigned> bad(nt, 0);
-  std::vector<std::thread> th;
   const size_t chunk = (n + nt - 1) / nt;
-  for (size_t t = 1; t < nt; t++)
-    th.emplace_back([&, t] { bad[t] = part(std::min(n, t * chunk), std::min(n, (t + 1) * chunk)); });
-  bad[0] = part(0, std::min(n, chunk));
-  unsigned any = bad[0];
-  for (size_t t = 1; t < nt; t++) {
-    th[t - 1].join();
-    any |= bad[t];
-  }
+  on_threads(nt, [&](size_t t) {
+    bad[t] = part(std::min(n, t * chunk), std::min(n, (t + 1) * chunk));
+  });
+  unsigned any = 0;
+  for (unsigned b : bad) any |= b;
   return any;
 }
 

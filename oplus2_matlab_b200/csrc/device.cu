@@ -17,6 +17,7 @@
 #include <unordered_set>
 #include <vector>
 
+#include "host_threads.h"
 #include "loops.h"
 
 void op2b_release_plans();  // plan.cu
@@ -412,17 +413,11 @@ static bool host_all_zero(const char *p, size_t n) {
   const size_t nt = hw < 2 ? 1 : std::min<size_t>(8, hw);
   const size_t chunk = (n - head + nt - 1) / nt;
   std::vector<char> zero(nt, 1);
-  std::vector<std::thread> th;
-  for (size_t t = 1; t < nt; t++)
-    th.emplace_back([&, t] {
-      zero[t] = part(std::min(n, head + t * chunk), std::min(n, head + (t + 1) * chunk));
-    });
-  zero[0] = part(head, std::min(n, head + chunk));
-  bool all = zero[0] != 0;
-  for (size_t t = 1; t < nt; t++) {
-    th[t - 1].join();
-    all = all && zero[t] != 0;
-  }
+  on_threads(nt, [&](size_t t) {
+    zero[t] = part(std::min(n, head + t * chunk), std::min(n, head + (t + 1) * chunk));
+  });
+  bool all = true;
+  for (char z : zero) all = all && z;
   return all;
 }
 

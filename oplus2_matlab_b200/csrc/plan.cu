@@ -23,6 +23,7 @@
 #include <cstring>
 #include <thread>
 
+#include "host_threads.h"
 #include "plan.h"
 
 namespace op2b {
@@ -2095,13 +2096,10 @@ static void *plan_slab(size_t bytes) {
   char *p = (char *)malloc(bytes ? bytes : 1);
   const size_t nt = std::min<size_t>(8, std::max(1u, std::thread::hardware_concurrency()));
   if (!p || bytes < ((size_t)4 << 20) || nt < 2) return p;
-  auto touch = [p](size_t a, size_t b) {
-    for (size_t i = a; i < b; i += 4096) static_cast<volatile char *>(p)[i] = 0;
-  };
-  std::vector<std::thread> th;
-  for (size_t t = 1; t < nt; t++) th.emplace_back(touch, bytes / nt * t, bytes / nt * (t + 1));
-  touch(0, bytes / nt);
-  for (auto &t : th) t.join();
+  on_threads(nt, [p, bytes, nt](size_t t) {
+    for (size_t i = bytes / nt * t; i < bytes / nt * (t + 1); i += 4096)
+      static_cast<volatile char *>(p)[i] = 0;
+  });
   return p;
 }
 
