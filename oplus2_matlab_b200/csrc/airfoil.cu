@@ -2011,29 +2011,30 @@ static ChainSched *chain_sched(SlotPlan *sp, int et, int ct, int lag) {
 }
 
 // the plans and value buffer of a res_calc (+ bres_calc) chain; nullptr
-// when the mesh does not suit slots, or when something is not there yet and
-// build is false; *err when a plan failed
+// when the mesh does not suit slots, or when `make` goes no further; *err
+// when a plan failed (Make::kBuild only)
 template <class T>
 static SlotPlan *chain_plans(op_set rset, const op_arg *ra, op_set bset, const op_arg *ba,
-                             bool *err, bool build = true) {
+                             bool *err, Make make) {
   *err = false;
-  GatherPlan *g = get_gather_plan(rset, ra, {6, 7}, build);
-  GatherPlan *gb = ba ? get_gather_plan(bset, ba, {4}, build) : nullptr;
+  GatherPlan *g = get_gather_plan(rset, ra, {6, 7}, make);
+  GatherPlan *gb = g && ba ? get_gather_plan(bset, ba, {4}, make) : nullptr;
   if (!g || (ba && !gb)) {
-    *err = build;
+    *err = make == Make::kBuild;
     return nullptr;
   }
-  SlotPlan *sp = get_slot_plan(g, gb, build);
+  SlotPlan *sp = get_slot_plan(g, gb, make);
   if (!sp) return nullptr;
   const size_t nval = (size_t)sp->na + sp->nb + 1;
   const size_t need = sizeof(T) * 4 * nval;
   if (sp->buf_bytes < need) {
-    if (!build) return nullptr;
+    if (make == Make::kFind) return nullptr;
     dev_free(sp->d_buf);
-    sp->d_buf = dev_alloc(need);
+    sp->d_buf = make == Make::kTry ? dev_try_alloc(need) : dev_alloc(need);
     sp->buf_bytes = sp->d_buf ? need : 0;
     if (!sp->d_buf) {
-      *err = true;
+      sp->no_room = true;
+      *err = make == Make::kBuild;
       return nullptr;
     }
     // the padding entry, never written by the flux pass: -0.0
@@ -2053,18 +2054,14 @@ static SlotPlan *chain_plans(op_set rset, const op_arg *ra, op_set bset, const o
 // block colours, each launch a chain of dependent steps over a quarter of the
 // blocks; 116 us so.
 // The block kernels remain for cells of more than kMaxSlotWidth
-// contributions, for bres_calc on its own, and in a capture of a loop whose
-// lists are not there yet.
+// contributions, for bres_calc on its own, where there is no room for the
+// lists or the values, and in a capture of a loop whose lists are not there
+// yet: COLOURED needs none of them.
 bool coloured_fold() { return tuning("coloured_fold", 1) && tuning("gather_slots", 1); }
 
-static const int *coloured_ell(SlotPlan *sp, const SlotPlan::Order *o, op_set rset,
-                               const op_arg *ra, op_set bset, const op_arg *ba,
-                               const ColourKey &key) {
-  DevPlan *p = get_plan(key.rname, rset, key.rpart, 8, ra, 4, kResInds);
-  DevPlan *pb = ba ? get_plan(key.bname, bset, key.bpart, 6, ba, 4, kBresInds) : nullptr;
-  if (!p || (ba && !pb)) return nullptr;
-  return get_coloured_lists(sp, o, p, key.rblock > 0 ? key.rblock : 512, pb,
-                            key.bblock > 0 ? key.bblock : 512);
+// how far a chain may go for its plans and lists
+static Make chain_make(bool col) {
+  return !col ? Make::kBuild : stream_capturing() ? Make::kFind : Make::kTry;
 }
 
 template <class T>
@@ -2098,7 +2095,9 @@ static bool res_flux_ahead_t(op_set rset, const op_arg *ra, op_set bset, const o
   AirConsts<T> K = air_consts<T>();
   if (error_pending()) return false;
   bool err = false;
-  SlotPlan *sp = chain_plans<T>(rset, ra, bset, ba, &err);
+  SlotPlan *sp =
+      chain_plans<T>(rset, ra, bset, ba, &err,
+                     chain_make(effective_strategy("res_calc") == OP2B_STRATEGY_COLOURED));
   if (!sp || err) return false;
   ResEdges<T> E = res_edges<T>(rset, ra);
   BresEdges<T> B = bres_edges<T>(bset, ba);
@@ -2694,11 +2693,22 @@ static bool res_chain_t(char const *loop_name, op_set rset, const op_arg *ra, op
   cudaStream_t s = rt().stream;
   bool err = false;
   const bool col = effective_strategy(key.rname) == OP2B_STRATEGY_COLOURED;
-  // a capture cannot make plans: COLOURED runs by block colours there unless
-  // all that its two passes need is there
-  SlotPlan *sp = chain_plans<T>(rset, ra, bset, ba, &err, !col || !stream_capturing());
+  // the colouring first: COLOURED cannot do without it
+  DevPlan *cp = nullptr, *cpb = nullptr;
+  if (col) {
+    if (!coloured_fold()) return false;
+    cp = get_plan(key.rname, rset, key.rpart, 8, ra, 4, kResInds);
+    if (cp && ba) cpb = get_plan(key.bname, bset, key.bpart, 6, ba, 4, kBresInds);
+    if (!cp || (ba && !cpb)) return true;
+  }
+  auto by_block_colours = [&]() {  // those find the plans again
+    if (cp) plan_unused(cp);
+    if (cpb) plan_unused(cpb);
+    return false;
+  };
+  SlotPlan *sp = chain_plans<T>(rset, ra, bset, ba, &err, chain_make(col));
   if (err) return true;
-  if (!sp) return false;
+  if (!sp) return by_block_colours();
   const int W = sp->width, ncell = sp->ntarget;
   const size_t nval = (size_t)sp->na + sp->nb + 1;
   T *vals = (T *)sp->d_buf;
@@ -2707,10 +2717,9 @@ static bool res_chain_t(char const *loop_name, op_set rset, const op_arg *ra, op
   if (error_pending()) return true;
   const int *ell = order ? order->d_ell : sp->d_ell;
   if (col) {
-    if (!coloured_fold()) return false;
-    ell = coloured_ell(sp, order, rset, ra, bset, ba, key);
-    if (error_pending()) return true;
-    if (!ell) return false;
+    ell = get_coloured_lists(sp, order, cp, key.rblock > 0 ? key.rblock : 512, cpb,
+                             key.bblock > 0 ? key.bblock : 512);
+    if (!ell) return by_block_colours();
   }
 
   std::string name = loop_name ? loop_name : "res_calc";

@@ -1336,6 +1336,11 @@ DevPlan *get_plan(char const *name, op_set set, int part_size, int nargs, const 
   return g_plans.back().get();
 }
 
+void plan_unused(DevPlan *p) {
+  p->count--;
+  p->pub.count = p->count;
+}
+
 long validate_plan(const DevPlan &p) {
   Runtime &R = rt();
   cudaStream_t s = R.stream;
@@ -1510,16 +1515,18 @@ __global__ void k_keys_through(int *keys, long long n, int nslots, const int *pe
 }
 
 GatherPlan *get_gather_plan(op_set set, const op_arg *args, const std::vector<int> &slots,
-                            bool build) {
+                            Make make) {
+  bool unsuited = false;
   for (auto &up : g_gather) {
     GatherPlan &g = *up;
     if (g.set != set || g.nslots != (int)slots.size() || g.dat != args[slots[0]].dat) continue;
     bool match = true;
     for (int k = 0; k < g.nslots && match; k++)
       match = g.maps[k] == args[slots[k]].map && g.idxs[k] == args[slots[k]].idx;
-    if (match) return &g;
+    if (match && !g.unsuited) return &g;
+    unsuited = unsuited || match;
   }
-  if (!build) return nullptr;
+  if (make == Make::kFind || (make == Make::kTry && unsuited)) return nullptr;
   Runtime &R = rt();
   cudaStream_t s = R.stream;
   std::unique_ptr<GatherPlan> up(new GatherPlan());
@@ -1544,35 +1551,57 @@ GatherPlan *get_gather_plan(op_set set, const op_arg *args, const std::vector<in
   }
   const int n = set->size, T = g.ntarget;
   const long long nkeys = (long long)n * g.nslots;
-  if (nkeys > INT_MAX) {
-    fail(-1, "op2b error -- loop too large for 32-bit gather keys\n");
+  int *mem = nullptr;  // scratch
+  auto give_up = [&]() -> GatherPlan * {
+    if (mem) OP2B_CUDA(cudaFreeAsync(mem, s));
+    dev_free(g.d_active);
+    dev_free(g.d_row);
+    dev_free(g.d_keys);
+    g.d_active = g.d_row = g.d_keys = nullptr;
+    if (make == Make::kTry) {
+      g.unsuited = true;
+      g_gather.push_back(std::move(up));
+    }
     return nullptr;
+  };
+  auto keep = [&](size_t ints) {
+    return (int *)(make == Make::kTry ? dev_try_alloc(sizeof(int) * ints)
+                                      : dev_alloc(sizeof(int) * ints));
+  };
+  if (nkeys > INT_MAX) {
+    if (make != Make::kTry) fail(-1, "op2b error -- loop too large for 32-bit gather keys\n");
+    return give_up();
   }
-  int *cnt = nullptr, *flags = nullptr, *pos = nullptr, *acnt = nullptr;
-  OP2B_CUDA(pool_malloc_async((void **)&cnt, sizeof(int) * T, s));
+  const size_t Tz = (size_t)T;
+  const cudaError_t room = pool_malloc_async((void **)&mem, sizeof(int) * (6 * Tz + 3), s);
+  if (room != cudaSuccess) {
+    mem = nullptr;
+    cudaGetLastError();
+    if (make != Make::kTry) OP2B_CUDA(room);
+    return give_up();
+  }
+  int *cnt = mem, *flags = cnt + Tz, *pos = flags + Tz, *acnt = pos + Tz, *cursor = acnt + Tz;
+  int *long_rows = cursor + Tz + 1, *nlong = long_rows + Tz, *maxlen = nlong + 1;
   OP2B_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * T, s));
   const int grid = R.num_sms * 8;
   k_gather_count<<<grid, 256, 0, s>>>(sm, g.nslots, n, cnt);
-  OP2B_CUDA(pool_malloc_async((void **)&flags, sizeof(int) * T, s));
-  OP2B_CUDA(pool_malloc_async((void **)&pos, sizeof(int) * T, s));
   k_flags<<<grid, 256, 0, s>>>(cnt, T, flags);
   g.nactive = (int)exclusive_scan(flags, pos, T, s);
   int *rowcnt = cnt;
   const int *slot_of_target = nullptr;
   if (g.nactive < T) {
-    g.d_active = (int *)dev_alloc(sizeof(int) * std::max(1, g.nactive));
-    OP2B_CUDA(pool_malloc_async((void **)&acnt, sizeof(int) * std::max(1, g.nactive), s));
+    g.d_active = keep(std::max(1, g.nactive));
+    if (!g.d_active) return give_up();
     k_compact_active<<<grid, 256, 0, s>>>(cnt, pos, T, g.d_active, acnt);
     rowcnt = acnt;
     slot_of_target = pos;
   }
-  g.d_row = (int *)dev_alloc(sizeof(int) * ((size_t)g.nactive + 1));
-  g.d_keys = (int *)dev_alloc(sizeof(int) * (size_t)std::max(1LL, nkeys));
+  g.d_row = keep((size_t)g.nactive + 1);
+  g.d_keys = keep((size_t)std::max(1LL, nkeys));
+  if (!g.d_row || !g.d_keys) return give_up();
   long long total = g.nactive ? exclusive_scan(rowcnt, g.d_row, g.nactive, s) : 0;
   int tot32 = (int)total;
   OP2B_CUDA(cudaMemcpyAsync(g.d_row + g.nactive, &tot32, sizeof(int), cudaMemcpyHostToDevice, s));
-  int *cursor = nullptr, *long_rows = nullptr, *nlong = nullptr, *maxlen = nullptr;
-  OP2B_CUDA(pool_malloc_async((void **)&cursor, sizeof(int) * ((size_t)g.nactive + 1), s));
   OP2B_CUDA(cudaMemcpyAsync(cursor, g.d_row, sizeof(int) * ((size_t)g.nactive + 1),
                             cudaMemcpyDeviceToDevice, s));
   k_gather_scatter<<<grid, 256, 0, s>>>(sm, g.nslots, n, slot_of_target, cursor, g.d_keys);
@@ -1581,18 +1610,17 @@ GatherPlan *get_gather_plan(op_set set, const op_arg *args, const std::vector<in
   const int *to_orig = perm_new2old_dev(set), *to_dev = perm_old2new_dev(set);
   if (to_orig && nkeys)
     k_keys_through<<<grid, 256, 0, s>>>(g.d_keys, nkeys, g.nslots, to_orig);
-  OP2B_CUDA(pool_malloc_async((void **)&long_rows, sizeof(int) * std::max(1, g.nactive), s));
-  OP2B_CUDA(pool_malloc_async((void **)&nlong, sizeof(int) * 2, s));
-  maxlen = nlong + 1;
   OP2B_CUDA(cudaMemsetAsync(nlong, 0, sizeof(int) * 2, s));
   k_sort_rows<<<grid, 256, 0, s>>>(g.d_row, g.nactive, g.d_keys, long_rows, nlong, maxlen);
   int h[2] = {0, 0};
   OP2B_CUDA(cudaMemcpyAsync(h, nlong, sizeof h, cudaMemcpyDeviceToHost, s));
   OP2B_CUDA(cudaStreamSynchronize(s));
   g.max_row = h[1];
+  if (make == Make::kTry && g.max_row > kMaxSlotWidth) return give_up();
   g.nkeys = total;
   g.ntiles = (int)((total + kTile - 1) / kTile);
-  g.d_tile_first = (int *)dev_alloc(sizeof(int) * ((size_t)g.ntiles + 1));
+  g.d_tile_first = keep((size_t)g.ntiles + 1);
+  if (!g.d_tile_first) return give_up();
   k_tile_first<<<(g.ntiles + 256) / 256, 256, 0, s>>>(g.d_row, g.nactive, g.ntiles, g.d_tile_first);
   if (h[0] > 0) {
     int P = 1;
@@ -1600,19 +1628,14 @@ GatherPlan *get_gather_plan(op_set set, const op_arg *args, const std::vector<in
     if ((size_t)P * sizeof(int) > smem_optin()) {
       fail(-1, "op2b error -- a target has %d contributions, too many to order on chip\n",
            g.max_row);
-      return nullptr;
+      dev_free(g.d_tile_first);
+      return give_up();
     }
     allow_smem(k_sort_long_rows);
     k_sort_long_rows<<<h[0], 1024, sizeof(int) * P, s>>>(g.d_row, long_rows, g.d_keys);
   }
   if (to_dev && nkeys) k_keys_through<<<grid, 256, 0, s>>>(g.d_keys, nkeys, g.nslots, to_dev);
-  OP2B_CUDA(cudaFreeAsync(cnt, s));
-  OP2B_CUDA(cudaFreeAsync(flags, s));
-  OP2B_CUDA(cudaFreeAsync(pos, s));
-  if (acnt) OP2B_CUDA(cudaFreeAsync(acnt, s));
-  OP2B_CUDA(cudaFreeAsync(cursor, s));
-  OP2B_CUDA(cudaFreeAsync(long_rows, s));
-  OP2B_CUDA(cudaFreeAsync(nlong, s));
+  OP2B_CUDA(cudaFreeAsync(mem, s));
   OP2B_CUDA(cudaStreamSynchronize(s));
   g_gather.push_back(std::move(up));
   return g_gather.back().get();
@@ -1677,10 +1700,16 @@ __global__ void __launch_bounds__(kOrderChunk)
 
 static std::vector<std::unique_ptr<SlotPlan>> g_slot_plans;
 
-SlotPlan *get_slot_plan(const GatherPlan *a, const GatherPlan *b, bool build) {
-  for (auto &up : g_slot_plans)
-    if (up->a == a && up->b == b) return up->width > 0 ? up.get() : nullptr;
-  if (!build) return nullptr;
+SlotPlan *get_slot_plan(const GatherPlan *a, const GatherPlan *b, Make make) {
+  for (auto it = g_slot_plans.begin(); it != g_slot_plans.end(); ++it) {
+    SlotPlan *p = it->get();
+    if (p->a != a || p->b != b) continue;
+    if (make != Make::kBuild) return p->width > 0 && !p->no_room ? p : nullptr;
+    if (p->width > 0 || !p->no_room) return p->width > 0 ? p : nullptr;
+    g_slot_plans.erase(it);  // there was no room before
+    break;
+  }
+  if (make == Make::kFind) return nullptr;
   std::unique_ptr<SlotPlan> up(new SlotPlan());
   SlotPlan &p = *up;
   p.a = a;
@@ -1694,7 +1723,15 @@ SlotPlan *get_slot_plan(const GatherPlan *a, const GatherPlan *b, bool build) {
     cudaStream_t s = rt().stream;
     const int grid = rt().num_sms * 8;
     int *cnt = nullptr;
-    OP2B_CUDA(pool_malloc_async((void **)&cnt, sizeof(int) * ((size_t)p.ntarget + 2), s));
+    const cudaError_t room =
+        pool_malloc_async((void **)&cnt, sizeof(int) * ((size_t)p.ntarget + 2), s);
+    if (room != cudaSuccess) {
+      cudaGetLastError();
+      if (make == Make::kBuild) OP2B_CUDA(room);
+      p.no_room = true;
+      g_slot_plans.push_back(std::move(up));
+      return nullptr;
+    }
     int *mx = cnt + p.ntarget;  // the longest list, the sample's lines
     OP2B_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * ((size_t)p.ntarget + 2), s));
     k_ell_count<<<grid, 256, 0, s>>>(a->nactive, a->d_active, a->d_row, cnt);
@@ -1721,9 +1758,11 @@ SlotPlan *get_slot_plan(const GatherPlan *a, const GatherPlan *b, bool build) {
     if (w >= 1 && w <= kMaxSlotWidth && (long long)w * p.ntarget <= 2 * nkeys + p.ntarget) {
       p.width = w;
       const size_t n = (size_t)w * p.ntarget;
-      p.d_ell = (int *)dev_alloc(sizeof(int) * n);
+      p.d_ell = (int *)(make == Make::kTry ? dev_try_alloc(sizeof(int) * n)
+                                           : dev_alloc(sizeof(int) * n));
       if (!p.d_ell) {
         p.width = 0;
+        p.no_room = true;
       } else {
         k_fill_int<<<grid, 256, 0, s>>>(p.d_ell, n, (p.na + p.nb) << 1);
         OP2B_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * (size_t)p.ntarget, s));
@@ -1789,8 +1828,11 @@ const int *get_coloured_lists(SlotPlan *sp, const SlotPlan::Order *o, const DevP
     if (c.o == o && c.p == p && c.pb == pb && c.nt == nt && c.nbt == nbt) return c.d_ell;
   if ((long long)sp->na + sp->nb + 1 >= (1LL << 29) || stream_capturing()) return nullptr;
   SlotPlan::Coloured c{p, pb, o, nt, nbt, nullptr};
-  c.d_ell = (int *)dev_alloc(sizeof(int) * (size_t)sp->width * sp->ntarget);
-  if (!c.d_ell) return nullptr;
+  c.d_ell = (int *)dev_try_alloc(sizeof(int) * (size_t)sp->width * sp->ntarget);
+  if (!c.d_ell) {
+    sp->no_room = true;
+    return nullptr;
+  }
   const ColouredLoop A{p->bsize, nt, p->d_blkcol, p->d_thrcol};
   const ColouredLoop B{pb ? pb->bsize : 1, nbt, pb ? pb->d_blkcol : nullptr,
                        pb ? pb->d_thrcol : nullptr};

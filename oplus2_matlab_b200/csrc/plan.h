@@ -66,7 +66,15 @@ struct GatherPlan {
   // first use (outside any graph capture) and kept with the plan
   void *d_contrib = nullptr;
   size_t contrib_bytes = 0;
+  bool unsuited = false;  // none of the arrays are there: Make::kTry gave up
 };
+
+// How far the finders of plans that a loop can do without may go: kFind returns
+// what is there (in a capture, which cannot make them); kTry makes it, but
+// reports no error and gives up, once and for all, on targets of more than
+// kMaxSlotWidth contributions and where there is no room; kBuild makes it or
+// reports an error.
+enum class Make { kFind, kTry, kBuild };
 
 // contributions per CTA tile of the contribution-parallel gather kernels
 constexpr int kTile = 256;
@@ -90,6 +98,7 @@ struct SlotPlan {
   int *d_ell = nullptr;     // [ntarget * width]
   void *d_buf = nullptr;    // the (na + nb + 1) values, allocated by the loop
   size_t buf_bytes = 0;
+  bool no_room = false;  // Make::kTry found no room for the lists or the values
   ChainSched *chain = nullptr;  // built by the first persistent chain launch
   bool chain_unsuited = false;  // a cell tile reads too many flux tiles for it
   // the edges of a in the order the flux pass takes them (get_flux_order)
@@ -121,8 +130,9 @@ void release_tile_plan(SlotPlan *sp);
 // strip of nt elements of the block, thread colour and slot, b's after a's;
 // entry index << 2 | last of its block << 1 | negate, -1 past the end.
 // o: when the flux pass has an order of its own.
-// Device memory kept with the slot plan; nullptr when the indices do not fit, or
-// when they are not there and a capture is under way, which cannot make them.
+// Device memory kept with the slot plan; nullptr when the indices do not fit,
+// when there is no room, or when they are not there and a capture is under way,
+// which cannot make them.
 const int *get_coloured_lists(SlotPlan *sp, const SlotPlan::Order *o, const DevPlan *p, int nt,
                               const DevPlan *pb, int nbt);
 
@@ -145,16 +155,17 @@ constexpr int kMaxSlotWidth = 8;
 // nullptr when some target has more than kMaxSlotWidth contributions or the
 // padding would more than double the lists (the caller then uses the CSR
 // fold).
-// (build false, here and for get_gather_plan: nullptr if it is not there yet)
-SlotPlan *get_slot_plan(const GatherPlan *a, const GatherPlan *b, bool build = true);
+SlotPlan *get_slot_plan(const GatherPlan *a, const GatherPlan *b, Make make = Make::kBuild);
 
 // Find or build the reference-compatible plan (device resident).
 DevPlan *get_plan(char const *name, op_set set, int part_size, int nargs, const op_arg *args,
                   int ninds, const int *inds);
+// the call that found it did not use it: op_plan's count of uses as before
+void plan_unused(DevPlan *p);
 // Find or build the gather plan for the INC args listed in slots (all on
 // the same dat).
 GatherPlan *get_gather_plan(op_set set, const op_arg *args, const std::vector<int> &slots,
-                            bool build = true);
+                            Make make = Make::kBuild);
 // Device validation of a plan; returns the number of violations.
 long validate_plan(const DevPlan &p);
 
