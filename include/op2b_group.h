@@ -112,8 +112,9 @@ int op2b_group_tiled(op2b_group g);
  * Results do not depend on it; op2b_group_autotune picks it by timing. */
 int op2b_group_set_edge_tile(op2b_group g, int edges_per_tile);
 int op2b_group_edge_tile(op2b_group g);
-/* Time `iters` iterations at each candidate edge tile, then at each block
- * size and stream count (one block on one stream; 96 or 48 MiB blocks on
+/* Time `iters` iterations (rounded up to the graphs of eight that a long run
+ * issues, and as many as no solve stops in) at each candidate edge tile, then
+ * at each block size and stream count (one block on one stream; 96 or 48 MiB blocks on
  * one stream; 48 or 24 MiB on two; 24 MiB on three; 12 MiB on four), on the
  * current active solves, putting their state back after each trial; keeps
  * the fastest of each and returns the edge tile. */

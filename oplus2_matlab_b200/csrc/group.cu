@@ -31,6 +31,7 @@
 // tables at the next op2b_group_run after a poll.
 
 #include <math.h>
+#include <limits.h>
 #include <string.h>
 
 #include <algorithm>
@@ -1304,6 +1305,20 @@ struct Group : GroupBase {
     if (changed) rebuild();
     if (nactive == 0 || iters <= 0) return etile;
     prime();  // before the snapshot: trials start from primed solves
+    // Timed as a long run issues them, kUnroll to a graph, and so that no
+    // solve reaches its cap in a trial: from there on its CTAs return at once,
+    // and every candidate looks alike.
+    int left = INT_MAX;
+    std::vector<SolveState> now(solves.size());
+    OP2B_CUDA(cudaMemcpyAsync(now.data(), d_st, sizeof(SolveState) * now.size(),
+                              cudaMemcpyDeviceToHost, cs));
+    OP2B_CUDA(cudaStreamSynchronize(cs));
+    for (size_t i = 0; i < solves.size(); i++)
+      if (solves[i].joined && !solves[i].removed && !solves[i].done && now[i].active)
+        left = std::min(left, now[i].max_iter - now[i].iter);
+    if (error_pending() || left == INT_MAX) return etile;
+    const int unit = left >= kUnroll ? kUnroll : 1;
+    const int timed = (int)std::min<long long>(left, (iters + unit - 1LL) / unit * unit) / unit * unit;
     // snapshot of everything an iteration writes
     std::vector<std::pair<void *, size_t>> regions;
     for (auto &s : solves) {
@@ -1335,10 +1350,11 @@ struct Group : GroupBase {
     OP2B_CUDA(cudaEventCreate(&e1));
     auto trial = [&]() {
       rebuild();
-      make_graphs(iters);
-      iterate(iters >= kUnroll ? kUnroll : 1);  // warm
+      make_graphs(unit);
+      iterate(unit);  // warm
+      copy(false);
       OP2B_CUDA(cudaEventRecord(e0, cs));
-      iterate(iters);
+      for (int i = 0; i < timed; i += unit) iterate(unit);
       OP2B_CUDA(cudaEventRecord(e1, cs));
       OP2B_CUDA(cudaEventSynchronize(e1));
       float ms = 0;
