@@ -257,6 +257,10 @@ unsigned long long op2b_tiled_launches(int reset);
  * res was known zero is set, at each launch, to read res when res may hold
  * other values then.  No counterpart in the reference. */
 unsigned long long op2b_res_skips(int reset);
+/* Orders of the flux pass (knob "flux_order") made since op_init, and in *kept
+ * (nullable) how many of them read fewer cells than the loop's own order and
+ * so are the one the pass takes.  Synchronises; -1 in a stream capture. */
+int op2b_flux_orders(int *kept);
 
 /* Bytes copied from host to device by dataset declarations and map uploads
  * since the last reset; reset != 0 clears the count.  A dataset declared

@@ -1874,7 +1874,7 @@ __global__ void k_order_lists(size_t n, int na, const int *__restrict__ ell,
                               const unsigned long long *__restrict__ cells,
                               const int2 *__restrict__ edge, const int2 *__restrict__ cell,
                               int4 *__restrict__ rows, int *__restrict__ out) {
-  const bool good = 4 * cells[0] < 3 * cells[1];
+  const bool good = 4 * cells[0] < 3 * cells[1];  // as flux_orders has it
   const size_t i0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = i0; i < n; i += stride) {
@@ -2012,13 +2012,11 @@ static void make_flux_order(SlotPlan *sp, SlotPlan::Order *o) {
   const int2 *cell = reinterpret_cast<const int2 *>(map_dev(o->mq));
   const size_t nlist = (size_t)sp->width * sp->ntarget;
   o->tried = true;
-  o->d_rows = (int4 *)dev_try_alloc(sizeof(int4) * (size_t)na + sizeof(int) * nlist);
-  o->d_ell = (int *)(o->d_rows + (o->d_rows ? na : 0));
-  // edges' places | distinct cells of a sample of the new order, of the old
-  int *mem = nullptr;
-  const size_t words = ((size_t)na + 1) / 2 * 2;
+  // rows | cells | lists
+  o->d_rows = (int4 *)dev_try_alloc(sizeof(int4) * ((size_t)na + 1) + sizeof(int) * nlist);
+  int *mem = nullptr;  // the edges' places
   bool good = o->d_rows &&
-              pool_malloc_async((void **)&mem, sizeof(int) * words + 16, s) == cudaSuccess;
+              pool_malloc_async((void **)&mem, sizeof(int) * (size_t)na, s) == cudaSuccess;
   if (good) {
     const int nnode = x->set->size;
     good = strcmp(x->type, "double") == 0
@@ -2026,7 +2024,8 @@ static void make_flux_order(SlotPlan *sp, SlotPlan::Order *o) {
                : coord_order(na, nnode, edge, cell, (const float *)x->data_d, o->d_rows, mem, s);
   }
   if (good) {
-    unsigned long long *cells = (unsigned long long *)(mem + words);
+    unsigned long long *cells = o->d_cells = (unsigned long long *)(o->d_rows + na);
+    o->d_ell = (int *)(o->d_rows + na + 1);
     const int step = (nchunk + 127) / 128, nsample = (nchunk + step - 1) / step;
     OP2B_CUDA(cudaMemsetAsync(cells, 0, 2 * sizeof *cells, s));
     k_chunk_cells<<<nsample, kOrderChunk, 0, s>>>(step, na, nullptr, o->d_rows, cells);
@@ -2038,7 +2037,6 @@ static void make_flux_order(SlotPlan *sp, SlotPlan::Order *o) {
     cudaGetLastError();
     dev_free(o->d_rows);
     o->d_rows = nullptr;
-    o->d_ell = nullptr;
   }
   if (mem) OP2B_CUDA(cudaFreeAsync(mem, s));
   if (!o->d_rows) return;
@@ -2067,6 +2065,23 @@ const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq, op_dat
   return o->d_rows ? o : nullptr;
 }
 
+int flux_orders(int *kept) {
+  int n = 0, k = 0;
+  if (kept) *kept = 0;
+  if (stream_capturing()) return -1;
+  for (auto &sp : g_slot_plans)
+    for (auto &o : sp->orders) {
+      if (!o->d_rows) continue;
+      unsigned long long c[2] = {0, 0};
+      OP2B_CUDA(cudaMemcpyAsync(c, o->d_cells, sizeof c, cudaMemcpyDeviceToHost, rt().stream));
+      OP2B_CUDA(cudaStreamSynchronize(rt().stream));
+      n++;
+      k += 4 * c[0] < 3 * c[1];
+    }
+  if (kept) *kept = k;
+  return n;
+}
+
 void make_flux_orders() {
   if (stream_capturing()) return;
   for (auto &sp : g_slot_plans)
@@ -2085,9 +2100,7 @@ void op2b_release_plans() {
     dev_free(up->d_ell);
     dev_free(up->d_buf);
     for (auto &c : up->coloured) dev_free(c.d_ell);
-    for (auto &o : up->orders) {
-      dev_free(o->d_rows);
-    }
+    for (auto &o : up->orders) dev_free(o->d_rows);
   }
   g_slot_plans.clear();
   for (auto &up : g_plans) {
@@ -2146,6 +2159,12 @@ static void *plan_slab(size_t bytes) {
 }
 
 extern "C" {
+
+int op2b_flux_orders(int *kept) {
+  op2b::flush_pending();
+  if (kept) *kept = 0;
+  return rt().cuda_ready ? flux_orders(kept) : 0;
+}
 
 op_plan *op_plan_get(char const *name, op_set set, int part_size, int nargs, op_arg *args,
                      int ninds, int *inds) {

@@ -107,6 +107,9 @@ struct SlotPlan {
     op_dat x = nullptr;                 // the nodes' coordinates
     int4 *d_rows = nullptr;  // [na] the edges' rows of them: two nodes, two cells
     int *d_ell = nullptr;    // the lists, with the places of the edges' values
+    // distinct cells of a sample of the order, and of the loop's own: rows and
+    // lists hold the loop's order where that is no better (k_order_lists)
+    unsigned long long *d_cells = nullptr;
     long long passes = 0;    // flux passes in the loop's order
     bool tried = false;
   };
