@@ -67,9 +67,10 @@ enum { OP2B_REDUCE_TREE = 0, OP2B_REDUCE_SEQ = 1 };
  *                   cell ahead of this cell's arithmetic; 0: the general pass
  *   "flux_order"    1 (default): where the numbering has no locality, the flux
  *                   pass of a mesh of 16,384 or more edges takes them in the
- *                   order of their nodes' coordinates, below a million edges
- *                   from the pass on by which making the order pays, or a
- *                   capture; 2: from the first pass; 0: in edge order
+ *                   order of their nodes' coordinates, from the pass on by
+ *                   which making the order has paid (the 21st to the 326th),
+ *                   or from a capture on; 2: from the first pass; 0: in edge
+ *                   order
  *   "red_tail"      1 (default): the rms of an update is folded by the flux
  *                   pass behind it, where the library issues that one too
  *                   (run ahead, or in a capture by op2b_capture_begin); 0: by

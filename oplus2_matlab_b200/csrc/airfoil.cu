@@ -1859,18 +1859,19 @@ static bool flux_pair_shape(const op_arg *ra, size_t nval) {
 }
 
 // the order the flux pass takes these edges in; nullptr: the loop's own.  next:
-// a pass is about to run, and may be the first in an order made for it.  Making
-// one costs what it saves in about 4 + 6M / edges passes (100 us and 17 us a
-// pass and million edges), so a mesh evaluated a few times does without: the
-// first nine evaluations of 21k cells in FP64 took 747 us with it, 649 without.
-// A million edges and more start with it, since ten passes are five iterations:
-// the first four of 2.88M cells 3.72 ms, 4.02 without it, 4.20 from the sixth
-// pass on.
+// a pass is about to run, and may be the first in an order made for it, after as
+// many passes as making it costs, so that no mesh loses more by it than it has
+// had to gain.  Cost and gain of a pass in FP32, the device pool holding the
+// memory: 60k edges 125 and 1.4 us (90 passes), 575k 155 and 6.5 (24; FP64 155
+// and 5: 31), 1.05M 182 and 7 (26), 1.3M 200 and 13.8 (15), 5.8M 525 to 1200
+// and 92 (6 to 13); where the pool has to map it first 180, 500, 550, 500 and
+// 1700 to 2500 us (19 to 28 passes at 5.8M, some 100 below).  20 + 5M / edges
+// lies between the two from 0.5M edges on, at the first of them below.
 static const SlotPlan::Order *flux_order(SlotPlan *sp, const op_arg *ra, bool next) {
   const int on = sp->scattered ? tuning("flux_order", 1) : 0;
   if (!on || !tuning("flux_pair", 1) || !flux_pair_shape(ra, (size_t)sp->na + sp->nb + 1))
     return nullptr;
-  const long long after = on == 2 || sp->na >= 1 << 20 ? 0 : 4 + 6000000 / std::max(sp->na, 1);
+  const long long after = on == 2 ? 0 : 20 + 5000000 / std::max(sp->na, 1);
   return get_flux_order(sp, ra[0].map, ra[2].map, ra[0].dat, next ? after : -1);
 }
 

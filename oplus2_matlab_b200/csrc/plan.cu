@@ -1855,8 +1855,9 @@ const int *get_coloured_lists(SlotPlan *sp, const SlotPlan::Order *o, const DevP
 // values in the same order.  (Coordinates are a guess -- res_calc's first
 // dataset, two reals per node -- and the order is dropped when a sample of it
 // is no better.)  A captured iteration of scrambled meshes: 720k FP32 cells 126 ->
-// 92 us, 2.88M 674 -> 471, 405k FP64 102 -> 81; the plan, about 0.5 ms of kernels
-// at 5.8M edges, is paid for by the first iterations.
+// 92 us, 2.88M 674 -> 471, 405k FP64 102 -> 81.  Making it takes about 0.5 ms of
+// kernels at 5.8M edges and 200 MB, whose mapping takes longer where the pool has
+// not got it: flux_order says from which pass on that pays.
 // A counting sort: the strips by a histogram of the first coordinate in 65,536
 // steps, then one bin per strip and step of the second.  Edges of one bin lie in
 // any order; the sums do not depend on it.

@@ -64,6 +64,18 @@ def test_made_and_kept(dt, n):
         assert a == b
 
 
+def test_made_once_it_has_paid():
+    """1.05M edges, knob 1: after 24 passes, two an iteration, whatever the
+    size above or below a million edges."""
+    mesh = M.naca0012(480, 366, scramble=True)
+    assert mesh.nedge > 1 << 20
+    a, _ = solve(mesh, np.float32, api.STRATEGY_GATHER, 0, 16)
+    for steps, want in ((4, (0, 0)), (10, (0, 0)), (16, (1, 1))):
+        b, made = solve(mesh, np.float32, api.STRATEGY_GATHER, 1, steps)
+        assert made == want, steps
+    assert a == b
+
+
 def test_numbering_with_locality():
     assert solve(with_edges(LEAST, scramble=False), np.float32, api.STRATEGY_GATHER, 2)[1] == (0, 0)
 
