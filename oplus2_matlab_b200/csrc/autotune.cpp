@@ -160,19 +160,20 @@ namespace op2b {
 namespace {
 
 // one launch of the chain as the dispatcher runs it with reductions
-// deferred (flux and fold, or the persistent launch) or loop by loop
-// (COLOURED by block colours); the reductions are left undelivered.  false: not applicable
+// deferred (flux and fold, or the persistent launch), or loop by loop
+// (COLOURED by block colours, where its two passes do not apply); the
+// reductions are left undelivered.  false: not applicable
 bool run_once(const ChainArgs &c, const Candidate &cand) {
-  if (cand.strategy == OP2B_STRATEGY_COLOURED && !coloured_fold()) {
+  std::vector<GblRequest> held;
+  const bool ok = run_res_chain(nullptr, c.rset, c.ra.data(), c.bset, c.ba.data(), c.ua.data(),
+                                c.aa.data(), nullptr, nullptr, nullptr, false, &held);
+  if (!ok && !error_pending() && cand.strategy == OP2B_STRATEGY_COLOURED) {
     run_res_calc("res_calc", c.rset, c.ra.data());
     run_bres_calc("bres_calc", c.bset, c.ba.data());
     run_airfoil_update("update", c.uset, c.ua.data());
     run_adt_calc("adt_calc", c.aset, c.aa.data());
     return !error_pending();
   }
-  std::vector<GblRequest> held;
-  const bool ok = run_res_chain(nullptr, c.rset, c.ra.data(), c.bset, c.ba.data(), c.ua.data(),
-                                c.aa.data(), nullptr, nullptr, nullptr, false, &held);
   return ok && !error_pending();
 }
 
