@@ -40,6 +40,7 @@
 
 #include "internal.h"
 #include "loops.h"
+#include "plan.h"
 
 namespace op2b {
 namespace {
@@ -290,6 +291,9 @@ extern "C" int op2b_autotune(const char *cache_path, int iters, int allow_reorde
   for (auto &kv : kDefaults) old_knobs.emplace_back(kv.first, tuning(kv.first.c_str(), kv.second));
   Snapshot snap;
   if (!snap.take({c.ua[1].dat, c.ua[2].dat, c.ua[3].dat, c.aa[5].dat})) return -1;
+  // the order that a long run's flux passes take, not made inside the one
+  // timed launch that reaches its number of passes
+  make_flux_orders();
   OP2B_CUDA(cudaStreamSynchronize(rt().stream));
   rt().error_mode = OP2B_ERRORS_RETURN;  // a failing candidate is skipped, not fatal
   std::vector<Candidate> cands = candidates(allow_reorder != 0);

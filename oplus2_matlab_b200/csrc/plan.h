@@ -148,8 +148,11 @@ const int *get_coloured_lists(SlotPlan *sp, const SlotPlan::Order *o, const DevP
 // listed in the order that it took, so only a caller about to run one may make it
 const SlotPlan::Order *get_flux_order(SlotPlan *sp, op_map mx, op_map mq, op_dat x,
                                       long long after);
-// at the start of a capture, which is replayed often and cannot make them
+// at the start of a capture, which is replayed often and cannot make them, and
+// of the autotuner's timings
 void make_flux_orders();
+// the orders made, and those that the sample kept (waits; -1 in a capture)
+int flux_orders(int *kept);
 
 // widest list the fold kernels accept
 constexpr int kMaxSlotWidth = 8;

@@ -6,6 +6,7 @@ import pytest
 
 from oplus2_matlab_b200 import api, apps
 from oplus2_matlab_b200 import mesh as M
+from test_autotune_gpu import DEFAULTS
 
 pytestmark = pytest.mark.gpu
 
@@ -31,5 +32,7 @@ def test_block_colours_are_a_candidate(op2, dt):
         api.sync()
         assert api.last_error() == ""
     finally:
+        for k, v in DEFAULTS.items():
+            lib.op2b_set_tuning(k.encode(), v)
         api._lib.global_int("OP_part_size").value = part
         api._lib.global_int("OP_block_size").value = block

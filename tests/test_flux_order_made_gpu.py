@@ -11,6 +11,7 @@ import pytest
 
 from oplus2_matlab_b200 import api, apps
 from oplus2_matlab_b200 import mesh as M
+from test_autotune_gpu import DEFAULTS
 
 pytestmark = pytest.mark.gpu
 
@@ -74,6 +75,19 @@ def test_made_once_it_has_paid():
         b, made = solve(mesh, np.float32, api.STRATEGY_GATHER, 1, steps)
         assert made == want, steps
     assert a == b
+
+
+def test_made_before_the_autotuner_times(op2):
+    api.set_strategy(api.STRATEGY_GATHER)
+    A = apps.Airfoil(with_edges(28500), np.float32)
+    A.iterate(1)
+    assert orders() == (0, 0)
+    try:
+        assert api.lib().op2b_autotune(None, 1, 0) == 0, api.last_error()
+        assert orders() == (1, 1)
+    finally:
+        for k, v in DEFAULTS.items():
+            api.lib().op2b_set_tuning(k.encode(), v)
 
 
 def test_numbering_with_locality():
