@@ -1865,8 +1865,8 @@ static bool flux_pair_shape(const op_arg *ra, size_t nval) {
 // memory: 60k edges 125 and 1.4 us (90 passes), 575k 155 and 6.5 (24; FP64 155
 // and 5: 31), 1.05M 182 and 7 (26), 1.3M 200 and 13.8 (15), 5.8M 525 to 1200
 // and 92 (6 to 13); where the pool has to map it first 180, 500, 550, 500 and
-// 1700 to 2500 us (19 to 28 passes at 5.8M, some 100 below).  20 + 5M / edges
-// lies between the two from 0.5M edges on, at the first of them below.
+// 1700 to 2500 us (19 to 28 passes at 5.8M, 47 at 1.3M, some 100 below).  20 + 5M /
+// edges lies at the first of the two numbers or between them.
 static const SlotPlan::Order *flux_order(SlotPlan *sp, const op_arg *ra, bool next) {
   const int on = sp->scattered ? tuning("flux_order", 1) : 0;
   if (!on || !tuning("flux_pair", 1) || !flux_pair_shape(ra, (size_t)sp->na + sp->nb + 1))

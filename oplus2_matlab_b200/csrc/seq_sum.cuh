@@ -26,7 +26,8 @@
 //
 // Bound: the walk's dependent steps (1-1.5 us for each of some 15 to 25 binade
 // changes of airfoil's rms) and reading the values twice.  720k values (180k
-// cells): 3.8 ms added one after another by one warp, about 50 us so.
+// cells): 3.8 ms added one after another by one warp, about 50 us so (FP64
+// about 90: 64-bit pairs, which spill at the 64 registers of 1024 threads).
 #pragma once
 
 #include <cuda_runtime.h>
