@@ -2085,9 +2085,18 @@ int flux_orders(int *kept) {
 
 void make_flux_orders() {
   if (stream_capturing()) return;
+  bool made = false;
   for (auto &sp : g_slot_plans)
     for (auto &o : sp->orders)
-      if (!o->d_rows && !o->tried) make_flux_order(sp.get(), o.get());
+      if (!o->d_rows && !o->tried) {
+        make_flux_order(sp.get(), o.get());
+        made = true;
+      }
+  if (!made) return;
+  // the launch behind, which would have to come after these (plan_queued), may be
+  // recorded and not run: the host waits instead
+  OP2B_CUDA(cudaStreamSynchronize(rt().stream));
+  rt().plan_queued = false;
 }
 
 }  // namespace op2b

@@ -76,6 +76,39 @@ def test_first_pass_of_a_rejected_order(dt):
     both(run)
 
 
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("noise", [False, True])
+def test_order_made_by_a_capture_that_is_not_launched(dt, noise):
+    """The loops recorded behind the making of the order run no kernel; the
+    next flux pass is an eager one (noise: its rows are the rejected order's)."""
+    mesh = M.naca0012(131, 77, scramble=True)
+    if noise:
+        mesh.x32 = np.random.default_rng(1).uniform(-1, 1, mesh.x32.shape).astype(np.float32)
+        mesh.x64 = mesh.x32.astype(np.float64)
+
+    def run():
+        lib = api.lib()
+        api.set_strategy(api.STRATEGY_GATHER)
+        A = apps.Airfoil(mesh, dt)
+        for nm in ("adt_calc", "res_calc", "bres_calc"):
+            A.loop(nm)
+        api.sync()
+        assert lib.op2b_flux_orders(None) == 0
+        assert lib.op2b_capture_begin(0) == 1, api.last_error()
+        for nm in ("adt_calc", "res_calc", "bres_calc"):
+            A.loop(nm)
+        h = lib.op2b_capture_end()
+        assert h, api.last_error()
+        for nm in ("res_calc", "bres_calc"):
+            A.loop(nm)
+        out = {k: v.copy() for k, v in A.fetch().items()}
+        assert lib.op2b_flux_orders(None) == 1
+        lib.op2b_graph_destroy(h)
+        return out
+
+    both(run)
+
+
 @pytest.mark.parametrize("variant", [1, 2])
 def test_pairs_are_not_made_in_a_capture(variant):
     """A capture's first res through another column of the map, then the same
