@@ -1572,8 +1572,9 @@ GatherPlan *get_gather_plan(op_set set, const op_arg *args, const std::vector<in
     if (make != Make::kTry) fail(-1, "op2b error -- loop too large for 32-bit gather keys\n");
     return give_up();
   }
-  const size_t Tz = (size_t)T;
-  const cudaError_t room = pool_malloc_async((void **)&mem, sizeof(int) * (6 * Tz + 3), s);
+  // parts on 16-byte boundaries: the scans read and write four values at once
+  const size_t Tz = ((size_t)T + 3) / 4 * 4;
+  const cudaError_t room = pool_malloc_async((void **)&mem, sizeof(int) * (6 * Tz + 6), s);
   if (room != cudaSuccess) {
     mem = nullptr;
     cudaGetLastError();
@@ -1581,7 +1582,7 @@ GatherPlan *get_gather_plan(op_set set, const op_arg *args, const std::vector<in
     return give_up();
   }
   int *cnt = mem, *flags = cnt + Tz, *pos = flags + Tz, *acnt = pos + Tz, *cursor = acnt + Tz;
-  int *long_rows = cursor + Tz + 1, *nlong = long_rows + Tz, *maxlen = nlong + 1;
+  int *long_rows = cursor + Tz + 4, *nlong = long_rows + Tz, *maxlen = nlong + 1;
   OP2B_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * T, s));
   const int grid = R.num_sms * 8;
   k_gather_count<<<grid, 256, 0, s>>>(sm, g.nslots, n, cnt);
